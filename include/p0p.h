@@ -44,7 +44,7 @@ enum {                                                                       /* 
 };
 /* which kernel family served the last p0p_gemm call (p0p_last_kernel) or is forced (p0p_gemm_args.force_kernel) */
 enum { P0P_K_AUTO = 0, P0P_K_GENERIC = 1, P0P_K_DECODE = 2, P0P_K_UMMA = 3,
-       /* p0p_attention: the warp-level kernel / the tensor-memory kernel (p0p_attn_args.kernel forces one of them) */
+       /* p0p_attention: the split-key kernel / the tensor-memory kernel (p0p_attn_args.kernel forces one of them) */
        P0P_K_ATTN_WARP = 16, P0P_K_ATTN_TMEM = 17 };
 
 enum { P0P_OPT_USE_STREAM = 1 };

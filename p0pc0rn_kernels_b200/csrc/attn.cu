@@ -39,15 +39,15 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
   DeviceGuard g(c->device);
   const uint32_t which = a->struct_size >= offsetof(p0p_attn_args, kernel) + sizeof(uint32_t) ? a->kernel : 0u;
   if (which != 0u && which != P0P_K_ATTN_WARP && which != P0P_K_ATTN_TMEM) return fail(c, -2, "attention: unknown kernel selector %u", which);
-  static DeviceOnce once[2];
+  static DeviceOnce once[4];        // tensor-memory kernel, split-key kernel with 1 / 2 / 4 row tiles
   // ---- tensor-memory kernel: two tiles of 128 queries per block.  Fewer than 128 queries per head leave most of a tile
-  // empty: those calls (decode steps) stay on the warp-level kernel, whose tile is 64 queries.
+  // empty: those calls (decode steps) go to the split-key kernel.
   if (which == P0P_K_ATTN_TMEM || (which == 0u && Lq >= 128u)) {
     if (!tmap_encoder()) return fail(c, -12, "attention: the driver offers no tensor-map encoder");
     const uint32_t ldv = (Lk + 7u) & ~7u;
     const uint64_t vt_bytes = (uint64_t)Hkv * 128u * ldv * 2u;
     if (int rc = ensure_scratch(c, vt_bytes)) return rc;
-    int rc = once[1].run(c->device, [&] { return (int)cudaFuncSetAttribute(k_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATC_SMEM); });
+    int rc = once[0].run(c->device, [&] { return (int)cudaFuncSetAttribute(k_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATC_SMEM); });
     if (rc) return cuda_fail(c, (cudaError_t)rc, "attention kernel attribute");
     CUtensorMap mq, mk, mv;
     if (!make_map_3d(&mq, p.Q, 128u, Lq, Hq, 128u, (uint64_t)Lq * 128u, 128u) || !make_map_3d(&mk, p.K, 128u, Lk, Hkv, 128u, (uint64_t)Lk * 128u, 128u) ||
@@ -67,9 +67,24 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
     c->last_kernel = P0P_K_ATTN_TMEM;
     return 0;
   }
-  int rc = once[0].run(c->device, [&] { return (int)cudaFuncSetAttribute(k_attn128, cudaFuncAttributeMaxDynamicSharedMemorySize, AT_SMEM); });
+  // ---- split-key kernel.  Row tiles per block: as few as hold the rows that share a kv head (fewer rows leave more warps to the
+  // keys), at most four.  Splits: enough blocks for two per SM, a key tile of 64 at least per block.
+  p.rows = Hq / Hkv * Lq;
+  const uint32_t wm = p.rows <= 16u ? 1u : p.rows <= 32u ? 2u : 4u, rbs = (p.rows + 16u * wm - 1u) / (16u * wm), sms = (uint32_t)c->prop.multiProcessorCount;
+  const uint32_t keys = a->mode == 0u ? Lk : a->mode == 1u ? std::min(Lk, std::min(Lq, nvalid)) : std::min(Lk, nvalid), nt = (keys + 63u) / 64u;
+  const uint64_t units = (uint64_t)Hkv * rbs;
+  uint32_t S = units >= 2u * sms || units > c->n_counters ? 1u : std::min<uint32_t>(nt, (uint32_t)(2u * sms / units));
+  p.tps = (nt + S - 1u) / S; p.S = S = (nt + p.tps - 1u) / p.tps;
+  if (S > 1u) {
+    const uint64_t slabs = units * S * 16u * wm;
+    if (int rc = ensure_scratch(c, slabs * (512u + 8u))) return rc;
+    p.part = reinterpret_cast<float*>(c->scratch); p.part_ml = reinterpret_cast<float2*>((char*)c->scratch + slabs * 512u); p.count = c->counters;
+  }
+  const auto kern = wm == 1u ? k_attn_split<1> : wm == 2u ? k_attn_split<2> : k_attn_split<4>;
+  int rc = once[wm == 4u ? 3 : wm].run(c->device, [&] { return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM); });
   if (rc) return cuda_fail(c, (cudaError_t)rc, "attention kernel attribute");
-  k_attn128<<<dim3((Lq + AT_BQ - 1) / AT_BQ, Hq), 128, AT_SMEM, c->stream>>>(p);
+  if (Hkv > 65535u || rbs > 65535u) return fail(c, -5, "attention: at most 65535 kv heads and 65535 blocks of query rows");
+  kern<<<dim3(S, Hkv, rbs), 128, AT_SMEM, c->stream>>>(p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(c, e, "attention launch");
   c->launches += 1;

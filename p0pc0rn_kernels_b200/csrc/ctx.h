@@ -39,6 +39,9 @@ struct p0p_ctx {
   // split-K partial sums of the decode kernel (grown on demand, owned by the context)
   void* scratch = nullptr;
   uint64_t scratch_bytes = 0;
+  // arrival counters of kernels whose last block finishes the work of the others: all zero between launches (that block resets its own)
+  uint32_t* counters = nullptr;
+  uint32_t n_counters = 0;
   bool capturing = false;
   std::unordered_set<void*> pinned;
   // a host-visible word kernels write when a bounded wait runs out (0 = fine)

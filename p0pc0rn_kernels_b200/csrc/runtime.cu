@@ -9,6 +9,8 @@ using namespace p0p;
 
 extern "C" {
 
+int p0p_close(p0p_ctx* c);
+
 uint32_t p0p_abi_version(void) { return P0P_ABI_VERSION; }
 
 int p0p_open(int device, const p0p_opts* opts, p0p_ctx** out) {
@@ -32,6 +34,9 @@ int p0p_open(int device, const p0p_opts* opts, p0p_ctx** out) {
     cudaEventDestroy(c->ev); if (c->own_stream) cudaStreamDestroy(c->stream); delete c; return (int)e;
   }
   *c->host_status = 0;
+  c->n_counters = 16384u;
+  if ((e = cudaMalloc((void**)&c->counters, c->n_counters * sizeof(uint32_t))) != cudaSuccess || (e = cudaMemsetAsync(c->counters, 0, c->n_counters * sizeof(uint32_t), c->stream)) != cudaSuccess ||
+      (e = cudaStreamSynchronize(c->stream)) != cudaSuccess) { p0p_close(c); return (int)e; }
   *out = c;
   return 0;
 }
@@ -73,6 +78,7 @@ int p0p_close(p0p_ctx* c) {
   c->bufs.clear();
   evict(c, 0);
   if (c->scratch) cudaFree(c->scratch);
+  if (c->counters) cudaFree(c->counters);
   if (c->host_status) cudaFreeHost(c->host_status);
   for (void* p : c->pinned) cudaFreeHost(p);
   cudaStreamSynchronize(c->stream);

@@ -85,3 +85,35 @@ def test_attention_errors(gpu):
     with pytest.raises(ValueError, match="multiple of Hkv"):
         P.attention(gpu, {"q": {"buf": b}, "k": {"buf": b}, "v": {"buf": b}, "o": {"buf": b}, "Lq": 1, "Lk": 1, "Hq": 3, "Hkv": 2})
     gpu.free(b)
+
+
+@pytest.mark.parametrize("Hq,Hkv,Lq,Lk,mode,nvalid", [
+    (4, 1, 4, 64, 0, 64),         # 16 packed rows: one full row tile, one key tile, no split
+    (17, 1, 1, 65, 0, 65),        # 17 rows: two row tiles, a last key tile of one key
+    (8, 2, 8, 700, 2, 641),       # 32 rows, splits whose last tile holds one valid key
+    (3, 1, 11, 1000, 2, 640),     # 33 rows: four row tiles, the last one with one row; splits that end on a tile's edge
+    (8, 1, 9, 2000, 2, 1999),     # 72 rows: two row blocks
+    (2, 2, 100, 300, 1, 90),      # causal: rows that see fewer keys than the first split holds, row blocks with their own key counts
+    (32, 8, 1, 4096, 2, 4000),    # a decoding step: 16 splits and more, merged by the last block
+])
+def test_attention_split_keys(gpu, oracle, Hq, Hkv, Lq, Lk, mode, nvalid):
+    """the split-key kernel of short query runs, at the edges of its row tiles, key tiles and splits; twice, so that a counter left
+    over from the first call would show"""
+    import p0pc0rn_kernels_b200 as P
+    O = oracle
+    Q = O.round_f16(O.randn(Hq * Lq * 128, 21, 0.5)); Kt = O.round_f16(O.randn(Hkv * Lk * 128, 22, 0.5)); V = O.round_f16(O.randn(Hkv * Lk * 128, 23))
+    want = O.cpu_attn(Q, Kt, V, Hq=Hq, Hkv=Hkv, Lq=Lq, Lk=Lk, mode=mode, nvalid=nvalid)
+    kh = P.toF16(Kt).reshape(Hkv, Lk, 128); vh = P.toF16(V).reshape(Hkv, Lk, 128)
+    if mode == 2: kh[:, nvalid:] = 0x7E01; vh[:, nvalid:] = 0x7E01                            # the unused end of a cache may hold anything, NaN too
+    qb, kb, vb = gpu.upload(P.toF16(Q)), gpu.upload(kh), gpu.upload(vh)
+    ob = gpu.buffer(Lq * Hq * 256)
+    try:
+        for _ in range(2):
+            gpu.upload(np.full(Lq * Hq * 128, 0x7E01, np.uint16), dst=ob)
+            P.attention(gpu, {"q": {"buf": qb}, "k": {"buf": kb}, "v": {"buf": vb}, "o": {"buf": ob}, "Lq": Lq, "Lk": Lk, "Hq": Hq, "Hkv": Hkv, "mode": mode, "nvalid": nvalid})
+            assert gpu.lastKernel == 16
+            got = P.fromF16(gpu.read(ob).view(np.uint16))
+            assert O.compare(got, want)[0] > 0.9995
+            assert np.abs(got - want).max() <= 2e-2 * np.abs(want).max()
+    finally:
+        for b in (qb, kb, vb, ob): gpu.free(b)
