@@ -44,16 +44,13 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
   // empty: those calls (decode steps) go to the split-key kernel.
   if (which == P0P_K_ATTN_TMEM || (which == 0u && Lq >= 128u)) {
     if (!tmap_encoder()) return fail(c, -12, "attention: the driver offers no tensor-map encoder");
-    const uint32_t ldv = (Lk + 7u) & ~7u;
-    const uint64_t vt_bytes = (uint64_t)Hkv * 128u * ldv * 2u;
-    if (int rc = ensure_scratch(c, vt_bytes)) return rc;
     int rc = once[0].run(c->device, [&] { return (int)cudaFuncSetAttribute(k_attn_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ATC_SMEM); });
     if (rc) return cuda_fail(c, (cudaError_t)rc, "attention kernel attribute");
     CUtensorMap mq, mk, mv;
-    if (!make_map_3d(&mq, p.Q, 128u, Lq, Hq, 128u, (uint64_t)Lq * 128u, 128u) || !make_map_3d(&mk, p.K, 128u, Lk, Hkv, 128u, (uint64_t)Lk * 128u, 128u) ||
-        !make_map_3d(&mv, c->scratch, Lk, 128u, Hkv, ldv, (uint64_t)ldv * 128u, 128u))
+    const uint32_t keys = a->mode ? std::min(Lk, nvalid) : Lk;      // (keys past the valid ones read as zero, whatever the buffer holds there)
+    if (!make_map_3d(&mq, p.Q, 128u, Lq, Hq, 128u, (uint64_t)Lq * 128u, 128u) || !make_map_3d(&mk, p.K, 128u, keys, Hkv, 128u, (uint64_t)Lk * 128u, 128u) ||
+        !make_map_3d(&mv, p.V, 128u, keys, Hkv, 128u, (uint64_t)Lk * 128u, 128u))
       return fail(c, -12, "attention: a tensor map could not be encoded");
-    k_attn_vt<<<dim3((Lk + 63u) / 64u, Hkv), 256, 0, c->stream>>>(p.V, reinterpret_cast<__half*>(c->scratch), Lk, ldv);
     AttnTcP t{};
     t.O = p.O; t.Lq = Lq; t.Lk = Lk; t.ldo = ldo; t.Hq = Hq; t.Hkv = Hkv; t.mode = a->mode; t.nvalid = nvalid; t.scale_log2 = p.scale_log2; t.status = c->dev_status;
     attn_plan(Lq, Lk, Hq, a->mode, nvalid, (uint32_t)c->prop.multiProcessorCount, t.np, t.ns);
@@ -63,7 +60,7 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
     k_attn_tc<<<Hq * (t.np + t.ns), ATC_THREADS, ATC_SMEM, c->stream>>>(t, mq, mk, mv);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(c, e, "attention launch");
-    c->launches += 2;
+    c->launches += 1;
     c->last_kernel = P0P_K_ATTN_TMEM;
     return 0;
   }

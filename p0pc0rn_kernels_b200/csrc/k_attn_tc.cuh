@@ -1,8 +1,9 @@
 // Flash attention, head_dim 128, on the 5th-generation tensor cores (src/ops/attention.js): the same contract as
-// k_attn.cuh (Q [Hq][Lq][128], K [Hkv][Lk][128] f16 head-major; O [Lq][ldo] token-major; mask modes 0 / 1 / 2; GQA), with
-// V given TRANSPOSED, [Hkv][128][ldv] (a pre-pass makes that copy), so that both products take K-major operands:
-//   S = Q K^T   A = Q tile [128 q][128 d] (shared memory),  B = K tile [128 keys][128 d] (shared memory)
-//   O += P V    A = P tile [128 q][128 keys] (tensor memory), B = V^T tile [128 d][128 keys] (shared memory)
+// k_attn.cuh (Q [Hq][Lq][128], K / V [Hkv][Lk][128] f16 head-major; O [Lq][ldo] token-major; mask modes 0 / 1 / 2; GQA):
+//   S = Q K^T   A = Q tile [128 q][128 d] (shared memory),  B = K tile [128 keys][128 d] (shared memory, K-major: d contiguous)
+//   O += P V    A = P tile [128 q][128 keys] (tensor memory), B = V tile [128 keys][128 d] (shared memory, MN-major: d, the N of
+//               this product, is contiguous).  V is read as it lies; a transposed copy (so that B would be K-major) was a pass of
+//               its own over V: ATTN_VT_NOTE
 // One block = two tiles of 128 queries of one head that share every K / V tile (or one tile: see attn_plan).  Tensor memory (512 columns x 128 lanes):
 // S of tile A | S of tile B | O of tile A | O of tile B, 128 fp32 columns each; lane = query row.  P (fp16, two keys per
 // column) is written over the first 64 columns of its S, which is free once the softmax threads hold the row.
@@ -22,11 +23,26 @@
 #include <functional>
 #include <vector>
 
+#include "epilogue.cuh"
 #include "sync.cuh"
 #include "umma.cuh"
 
 namespace p0p {
 
+__device__ __forceinline__ bool mbar_test(uint32_t bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile("{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool mbar_spin(uint32_t bar, uint32_t parity, int* status, int code) {
+  if (mbar_test(bar, parity)) return true;
+  const long long t0 = clock64();
+  uint32_t n = 0;
+  while (!mbar_test(bar, parity)) {
+    if ((++n & 255u) == 0u && clock64() - t0 > WAIT_LIMIT_CYCLES) { if (status) atomicCAS(status, 0, code); return false; }
+  }
+  return true;
+}
 struct AttnTcP {
   __half* O;
   uint32_t Lq, Lk, ldo, Hq, Hkv, mode, nvalid;
@@ -38,8 +54,8 @@ struct AttnTcP {
 #ifndef ATC_SLOTS_N
 #define ATC_SLOTS_N 4
 #endif
-constexpr uint32_t ATC_THREADS = 320u, ATC_TILE = 32768u, ATC_SLOTS = ATC_SLOTS_N;
-constexpr uint32_t ATC_SMEM = 1024u + (2u + ATC_SLOTS) * ATC_TILE + 256u;      // alignment slack + Q tiles + ring + barriers
+constexpr uint32_t ATC_THREADS = 576u, ATC_TILE = 32768u, ATC_SLOTS = ATC_SLOTS_N;
+constexpr uint32_t ATC_SMEM = 1024u + (2u + ATC_SLOTS) * ATC_TILE + 256u + 4096u;      // alignment slack + Q tiles + ring + barriers + the half rows' exchange
 
 #ifndef ATC_EMU
 #define ATC_EMU 6          // of every 16 pairs of scores, how many take their exponential on the FMA pipe instead of the MUFU
@@ -70,7 +86,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
   unsigned char* gbase = atc_raw + (base - smem_u32(atc_raw));
   const uint32_t q_sm = base, kv_sm = base + 2u * ATC_TILE, bars = kv_sm + ATC_SLOTS * ATC_TILE;
   const uint32_t q_full = bars, kv_full = bars + 8u, kv_empty = kv_full + 8u * ATC_SLOTS, s_full = kv_empty + 8u * ATC_SLOTS;
-  const uint32_t p_full = s_full + 16u, o_full = p_full + 32u, tmem_slot = o_full + 16u;      // p_full: [tile][half of the keys]
+  const uint32_t p_full = s_full + 16u, o_full = p_full + 16u, tmem_slot = o_full + 16u;
+  float* xch = reinterpret_cast<float*>(gbase + (bars + 256u - base));
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
   // the grid: first every head's two-tile blocks, then every head's one-tile blocks (the short ones fill the last wave)
   const bool hasB = blockIdx.x < p.Hq * p.np;
@@ -86,7 +103,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
   if (tid == 0) {
     mbar_init(q_full, 1u);
     for (uint32_t s = 0; s < ATC_SLOTS; s++) { mbar_init(kv_full + 8u * s, 1u); mbar_init(kv_empty + 8u * s, 1u); }
-    for (uint32_t t = 0; t < 2u; t++) { mbar_init(s_full + 8u * t, 1u); mbar_init(p_full + 16u * t, 4u); mbar_init(p_full + 16u * t + 8u, 4u); mbar_init(o_full + 8u * t, 1u); }
+    for (uint32_t t = 0; t < 2u; t++) { mbar_init(s_full + 8u * t, 1u); mbar_init(p_full + 8u * t, 8u); mbar_init(o_full + 8u * t, 1u); }
     fence_mbar_init();
   }
   if (warp == 1) { tmem_alloc(tmem_slot, 512u); tmem_relinquish(); }
@@ -105,13 +122,13 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
         const uint32_t slot = i % ATC_SLOTS, use = i / ATC_SLOTS, j = i >> 1, dst = kv_sm + slot * ATC_TILE, bar = kv_full + 8u * slot;
         if (use > 0u && !mbar_wait(kv_empty + 8u * slot, (use - 1u) & 1u, p.status, 401, 100u)) break;
         mbar_expect_tx(bar, ATC_TILE);
-        if (i & 1u) { for (uint32_t c = 0; c < 2u; c++) tma_load_3d(dst + c * 16384u, &mapV, (int)(j * 128u + c * 64u), 0, (int)hk, bar); }
+        if (i & 1u) { for (uint32_t c = 0; c < 2u; c++) tma_load_3d(dst + c * 16384u, &mapV, (int)(c * 64u), (int)(j * 128u), (int)hk, bar); }
         else { for (uint32_t c = 0; c < 2u; c++) tma_load_3d(dst + c * 16384u, &mapK, (int)(c * 64u), (int)(j * 128u), (int)hk, bar); }
       }
     }
   } else if (warp == 1) {
     // ================================================================= multiplies (the whole warp walks the loop, one lane issues)
-    const uint32_t idesc = umma_idesc_f16(128u, 128u), nt = hasB ? 2u : 1u;
+    const uint32_t idesc = umma_idesc_f16(128u, 128u), idesc_v = idesc | UMMA_B_MN, nt = hasB ? 2u : 1u;
     const uint64_t qd[2] = {umma_desc_sw128(q_sm), umma_desc_sw128(q_sm + ATC_TILE)};
     bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0u, p.status, 402) && mbar_wait(kv_full, 0u, p.status, 403));
     if (ok) {
@@ -133,23 +150,15 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
       bool rdy = mbar_wait(kv_full + 8u * sv, (iv / ATC_SLOTS) & 1u, p.status, 404);
       if (more) rdy = rdy && mbar_wait(kv_full + 8u * sk, (ik / ATC_SLOTS) & 1u, p.status, 405);
       if (!__all_sync(0xffffffffu, rdy)) { ok = false; break; }
-      const uint64_t vd = umma_desc_sw128(kv_sm + sv * ATC_TILE), kd = umma_desc_sw128(kv_sm + sk * ATC_TILE);
+      const uint64_t vd = umma_desc_sw128_mn(kv_sm + sv * ATC_TILE, 16384u), kd = umma_desc_sw128(kv_sm + sk * ATC_TILE);
       for (uint32_t t = 0; t < nt; t++) {
-        // P arrives in two halves of 64 keys: the first four multiplies of PV run while the second half's exponentials are computed
-        if (!__all_sync(0xffffffffu, mbar_wait(p_full + 16u * t, j & 1u, p.status, 406))) { ok = false; break; }
+        if (!__all_sync(0xffffffffu, mbar_spin(p_full + 8u * t, j & 1u, p.status, 406))) { ok = false; break; }
         tc_fence_after();
         const uint32_t s_col = tmem_base + t * 128u, o_col = tmem_base + 256u + t * 128u;
         const uint64_t qdt = qd[t];
         if (elect_one()) {
 #pragma unroll
-          for (uint32_t kk = 0; kk < 4u; kk++) umma_f16_ts(o_col, s_col + 8u * kk, vd + 2u * kk, idesc, j | kk);
-        }
-        __syncwarp();
-        if (!__all_sync(0xffffffffu, mbar_wait(p_full + 16u * t + 8u, j & 1u, p.status, 409))) { ok = false; break; }
-        tc_fence_after();
-        if (elect_one()) {
-#pragma unroll
-          for (uint32_t kk = 4u; kk < 8u; kk++) umma_f16_ts(o_col, s_col + 8u * kk, vd + 1024u + 2u * (kk & 3u), idesc, 1u);
+          for (uint32_t kk = 0; kk < 8u; kk++) umma_f16_ts(o_col, s_col + 8u * kk, vd + 128u * kk, idesc_v, j | kk);      // 16 keys further: 2048 bytes
           if (more) {
 #pragma unroll
             for (uint32_t kk = 0; kk < 8u; kk++) umma_f16_ss(s_col, qdt + (kk >> 2) * 1024u + 2u * (kk & 3u), kd + (kk >> 2) * 1024u + 2u * (kk & 3u), idesc, kk);
@@ -166,10 +175,13 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
       __syncwarp();
     }
   } else {
-    // ================================================================= softmax of one tile: thread = query row
-    const uint32_t t = (warp - 2u) >> 2, qd = warp & 3u, row = qd * 32u + lane, i = q0 + t * 128u + row;
+    // ================================================================= softmax of one tile: two threads per query row, 64 keys each
+    const uint32_t t = (warp - 2u) >> 3, half = ((warp - 2u) >> 2) & 1u, qd = warp & 3u, row = qd * 32u + lane, i = q0 + t * 128u + row;
     if (t == 0u || hasB) {
-      const uint32_t lane_addr = tmem_base + ((qd * 32u) << 16), s_addr = lane_addr + t * 128u, o_addr = lane_addr + 256u + t * 128u;
+      const uint32_t lane_addr = tmem_base + ((qd * 32u) << 16), s_addr = lane_addr + t * 128u + half * 64u, p_addr = lane_addr + t * 128u + half * 32u;
+      const uint32_t o_addr = lane_addr + 256u + t * 128u + half * 64u, pair_bar = 1u + t * 4u + qd;
+      // [parity of the key tile][tile][half][row]: what this thread tells its partner (row maximum; at the end, row sum)
+      float* mine = xch + (t * 2u + half) * 128u + row; const float* other = xch + (t * 2u + (half ^ 1u)) * 128u + row;
       uint32_t limit = p.Lk;                                                                  // keys [0, limit) are visible to this row
       if (p.mode == 1u) limit = min(p.Lk, min(i, p.nvalid - 1u) + 1u);
       if (p.mode == 2u) limit = min(p.Lk, p.nvalid);
@@ -177,32 +189,36 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
       float m_used = -INFINITY, l = 0.0f;
       bool ok = true;
       for (uint32_t j = 0; j < nj; j++) {
-        if (!mbar_wait(s_full + 8u * t, j & 1u, p.status, 407)) { ok = false; break; }
+        // (a wait that ran out: the thread goes on without it, so that its partner is not left at the barrier; the status word is set)
+        if (ok && !mbar_spin(s_full + 8u * t, j & 1u, p.status, 407)) ok = false;
         tc_fence_after();
-        uint32_t s[128];
+        uint32_t s[64];
 #pragma unroll
-        for (int c = 0; c < 8; c++) tmem_ld16(s_addr + 16u * c, *reinterpret_cast<uint32_t(*)[16]>(&s[16 * c]));
+        for (int c = 0; c < 4; c++) tmem_ld16(s_addr + 16u * c, *reinterpret_cast<uint32_t(*)[16]>(&s[16 * c]));
         tmem_ld_wait();
-        const int rel = (int)limit - (int)(j * 128u);                                         // columns [0, rel) of this tile are visible
-        if (__any_sync(0xffffffffu, rel < 128)) {
+        const int rel = (int)limit - (int)(j * 128u + half * 64u);                            // columns [0, rel) of this half are visible
+        if (__any_sync(0xffffffffu, rel < 64)) {
 #pragma unroll
-          for (int c = 0; c < 128; c++) s[c] = c < rel ? s[c] : 0xff800000u;
+          for (int c = 0; c < 64; c++) s[c] = c < rel ? s[c] : 0xff800000u;
         }
         float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-        for (int c = 0; c < 128; c += 4) {
+        for (int c = 0; c < 64; c += 4) {
           mx[0] = fmaxf(mx[0], __uint_as_float(s[c])); mx[1] = fmaxf(mx[1], __uint_as_float(s[c + 1]));
           mx[2] = fmaxf(mx[2], __uint_as_float(s[c + 2])); mx[3] = fmaxf(mx[3], __uint_as_float(s[c + 3]));
         }
-        const float mts = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3])) * sc;
+        float mts = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
+        mine[(j & 1u) * 512u] = mts;
+        bar_sync_named((int)pair_bar, 64);
+        mts = fmaxf(mts, other[(j & 1u) * 512u]) * sc;
         if (__any_sync(0xffffffffu, mts > m_used + 8.0f)) {
-          // raise the reference maximum of the whole warp's rows; O and l are rescaled to it
+          // raise the reference maximum of the warp's rows (its partner has the same rows and decides alike); O and l are rescaled to it
           const float m_new = fmaxf(m_used, mts);
           const float alpha = m_new == -INFINITY ? 1.0f : atc_ex2(m_used - m_new);
           l *= alpha;
           if (j > 0u) {
 #pragma unroll 1
-            for (uint32_t c = 0; c < 8u; c++) {
+            for (uint32_t c = 0; c < 4u; c++) {
               uint32_t o[16];
               tmem_ld16(o_addr + 16u * c, o);
               tmem_ld_wait();
@@ -216,7 +232,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
         float2 ls[2] = {make_float2(0.0f, 0.0f), make_float2(0.0f, 0.0f)};
         const float2 sc2 = make_float2(sc, sc), nm2 = make_float2(-m_used, -m_used);
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
+        for (int c = 0; c < 2; c++) {
           uint32_t pk[16];
 #pragma unroll
           for (int e = 0; e < 16; e++) {
@@ -228,24 +244,25 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
             const __half2 hp = __floats2half2_rn(pr.x, pr.y);
             pk[e] = *reinterpret_cast<const uint32_t*>(&hp);
           }
-          tmem_st16(s_addr + 16u * c, pk);
-          if (c == 1 || c == 3) {                                   // a half of P (64 keys) is complete: hand it to the multiplies
-            tmem_st_wait();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(p_full + 16u * t + (c == 3 ? 8u : 0u));
-          }
+          tmem_st16(p_addr + 16u * c, pk);
         }
+        tmem_st_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full + 8u * t);
         l += (ls[0].x + ls[0].y) + (ls[1].x + ls[1].y);
       }
+      mine[(nj & 1u) * 512u] = l;
+      bar_sync_named((int)pair_bar, 64);
+      l += other[(nj & 1u) * 512u];
       // ---- O / l -> global, token-major, head h at column h * 128
       if (ok && mbar_wait(o_full + 8u * t, 0u, p.status, 408)) {
         tc_fence_after();
         const float inv = 1.0f / l;
-        __half* dst = p.O + (size_t)i * p.ldo + h * 128u;
+        __half* dst = p.O + (size_t)i * p.ldo + h * 128u + half * 64u;
         const bool vec = ((reinterpret_cast<uintptr_t>(p.O) | ((uintptr_t)p.ldo * 2u)) & 15u) == 0u;
 #pragma unroll 1
-        for (uint32_t c = 0; c < 8u; c++) {
+        for (uint32_t c = 0; c < 4u; c++) {
           uint32_t o[16], w[8];
           tmem_ld16(o_addr + 16u * c, o);
           tmem_ld_wait();
@@ -301,27 +318,6 @@ inline void attn_plan(uint32_t Lq, uint32_t Lk, uint32_t Hq, uint32_t mode, uint
     if (span < best * 0.995) { best = span; np = n2; ns = s; }
   }
   std::copy(key, key + 6, memo.v); memo.np = np; memo.ns = ns;
-}
-
-// V [Hkv][Lk][128] -> V^T [Hkv][128][ldv] (ldv >= Lk, a multiple of 8): 64 keys x 128 dims per block through shared memory
-__global__ void __launch_bounds__(256) k_attn_vt(const __half* __restrict__ V, __half* __restrict__ Vt, uint32_t Lk, uint32_t ldv) {
-  __shared__ __half tile[64][130];
-  const uint32_t hk = blockIdx.y, k0 = blockIdx.x * 64u, tid = threadIdx.x;
-  const __half* src = V + (size_t)hk * Lk * 128u;
-  for (uint32_t e = tid; e < 64u * 64u; e += 256u) {             // 64 keys x 64 pairs of dims
-    const uint32_t r = e >> 6, c = e & 63u;
-    const uint32_t v = k0 + r < Lk ? __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)(k0 + r) * 128u) + c) : 0u;
-    *reinterpret_cast<uint32_t*>(&tile[r][2u * c]) = v;
-  }
-  __syncthreads();
-  __half* dst = Vt + (size_t)hk * 128u * ldv;
-  for (uint32_t e = tid; e < 128u * 32u; e += 256u) {            // 128 dims x 32 pairs of keys
-    const uint32_t d = e >> 5, kp = e & 31u, k = k0 + 2u * kp;
-    if (k < ldv) {                                                // ldv is even: the pair is inside the row
-      const __half2 o = __halves2half2(tile[2u * kp][d], tile[2u * kp + 1u][d]);
-      *reinterpret_cast<__half2*>(dst + (size_t)d * ldv + k) = o;
-    }
-  }
 }
 
 }  // namespace p0p

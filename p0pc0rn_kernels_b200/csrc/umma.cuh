@@ -25,6 +25,13 @@ __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::
 __device__ __forceinline__ uint64_t umma_desc_sw128(uint32_t smem_addr) {
   return (uint64_t)((smem_addr & 0x3ffffu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
+// ---- the same for an MN-major tile: rows of 64 fp16 along M / N (128 bytes, 128-byte swizzle), one row per k; the next 64 of M / N
+// lie `mn_stride` bytes further (the leading byte offset), the next 8 k 1024 bytes further (the stride byte offset).  16 k further:
+// start address + 2048 bytes.  Needs the operand's major bit in the instruction descriptor (UMMA_B_MN).
+__device__ __forceinline__ uint64_t umma_desc_sw128_mn(uint32_t smem_addr, uint32_t mn_stride) {
+  return (uint64_t)((smem_addr & 0x3ffffu) >> 4) | ((uint64_t)(mn_stride >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
+}
+constexpr uint32_t UMMA_B_MN = 1u << 16;
 // ---- instruction descriptor, kind::f16: fp16 A and B (K-major both), fp32 accumulate, M x N tile
 //   bits 4..5 D format (1 = f32)   7..9 A format (0 = f16)   10..12 B format (0 = f16)   15 / 16 A / B major (0 = K)
 //   bits 17..22 N >> 3             24..28 M >> 4
