@@ -3,7 +3,7 @@
 //   S = Q K^T   A = Q tile [128 q][128 d] (shared memory),  B = K tile [128 keys][128 d] (shared memory, K-major: d contiguous)
 //   O += P V    A = P tile [128 q][128 keys] (tensor memory), B = V tile [128 keys][128 d] (shared memory, MN-major: d, the N of
 //               this product, is contiguous).  V is read as it lies; a transposed copy (so that B would be K-major) was a pass of
-//               its own over V: ATTN_VT_NOTE
+//               its own over V (32:8 heads, 1000 causal tokens: 26.7 -> 24.6 us a call without it)
 // One block = two tiles of 128 queries of one head that share every K / V tile (or one tile: see attn_plan).  Tensor memory (512 columns x 128 lanes):
 // S of tile A | S of tile B | O of tile A | O of tile B, 128 fp32 columns each; lane = query row.  P (fp16, two keys per
 // column) is written over the first 64 columns of its S, which is free once the softmax threads hold the row.
@@ -88,7 +88,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
   const uint32_t q_full = bars, kv_full = bars + 8u, kv_empty = kv_full + 8u * ATC_SLOTS, s_full = kv_empty + 8u * ATC_SLOTS;
   const uint32_t p_full = s_full + 16u, o_full = p_full + 16u, tmem_slot = o_full + 16u;
   float* xch = reinterpret_cast<float*>(gbase + (bars + 256u - base));
-  const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
+  // (warp index and tensor-memory base through a shuffle: warp-uniform for the compiler, see k_umma.cuh)
+  const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31u;
   // the grid: first every head's two-tile blocks, then every head's one-tile blocks (the short ones fill the last wave)
   const bool hasB = blockIdx.x < p.Hq * p.np;
   const uint32_t b1 = blockIdx.x - p.Hq * p.np;
@@ -110,7 +111,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base));
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base)), 0);
 
   if (warp == 0) {
     // ================================================================= loads
