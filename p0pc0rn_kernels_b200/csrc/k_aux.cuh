@@ -60,31 +60,52 @@ inline cudaError_t launch_dequant(uint32_t enc, const uint8_t* W, uint32_t wG, u
 
 // ST[r*2] = (mean, rstd): mode 0 LayerNorm (mean removed), 1 RMS (mean = 0).  One block per row, fp32 sums,
 // two passes like the reference kernel (mean first, then squared deviations).
+// VEC: 16-byte loads of a row of up to 8192 columns that stays in the block's registers, so that memory is read once and all of a
+// thread's loads are in flight together.  Otherwise (odd alignment, longer rows) the row is read column by column, twice for
+// LayerNorm.  (3600 rows of 3072: 13.8 -> 12.6 us)
+template <bool VEC>
 __global__ void __launch_bounds__(256) k_rowstats(const float* __restrict__ X, uint32_t ld, uint32_t c0, uint32_t cols, uint32_t mode, float eps, float* __restrict__ ST) {
-  __shared__ float red[8];
+  __shared__ float red[2][8];
   const uint32_t row = blockIdx.x, t = threadIdx.x;
   const float* x = X + (size_t)row * ld + c0;
-  auto block_sum = [&](float v) -> float {
+  auto block_sum = [&](float v, uint32_t which) -> float {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    __syncthreads();
-    if ((t & 31u) == 0) red[t >> 5] = v;
+    if ((t & 31u) == 0) red[which][t >> 5] = v;
     __syncthreads();
     float s = 0.0f;
 #pragma unroll
-    for (int i = 0; i < 8; i++) s += red[i];
+    for (int i = 0; i < 8; i++) s += red[which][i];
     return s;
   };
-  float mean = 0.0f;
-  if (mode == 0u) { float s = 0.0f; for (uint32_t i = t; i < cols; i += 256u) s += x[i]; mean = block_sum(s) / (float)cols; }
-  float q = 0.0f;
-  for (uint32_t i = t; i < cols; i += 256u) { const float d = x[i] - mean; q = fmaf(d, d, q); }
-  const float var = block_sum(q) / (float)cols;
+  float mean = 0.0f, q = 0.0f;
+  if (VEC) {
+    float4 v[8];
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) { const uint32_t k = (i * 256u + t) * 4u; v[i] = k < cols ? __ldg(reinterpret_cast<const float4*>(x + k)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+    if (mode == 0u) {
+      float s = 0.0f;
+#pragma unroll
+      for (int i = 0; i < 8; i++) s += (v[i].x + v[i].y) + (v[i].z + v[i].w);
+      mean = block_sum(s, 0u) / (float)cols;
+    }
+#pragma unroll
+    for (uint32_t i = 0; i < 8u; i++) {
+      if ((i * 256u + t) * 4u >= cols) break;
+      const float dx = v[i].x - mean, dy = v[i].y - mean, dz = v[i].z - mean, dw = v[i].w - mean;
+      q += fmaf(dx, dx, dy * dy) + fmaf(dz, dz, dw * dw);
+    }
+  } else {
+    if (mode == 0u) { float s = 0.0f; for (uint32_t i = t; i < cols; i += 256u) s += x[i]; mean = block_sum(s, 0u) / (float)cols; }
+    for (uint32_t i = t; i < cols; i += 256u) { const float d = x[i] - mean; q = fmaf(d, d, q); }
+  }
+  const float var = block_sum(q, 1u) / (float)cols;
   if (t == 0) { ST[(size_t)row * 2u] = mean; ST[(size_t)row * 2u + 1u] = rsqrtf(var + eps); }
 }
 
 inline cudaError_t launch_rowstats(const float* X, uint32_t ld, uint32_t c0, uint32_t rows, uint32_t cols, uint32_t mode, float eps, float* ST, cudaStream_t st) {
-  k_rowstats<<<rows, 256, 0, st>>>(X, ld, c0, cols, mode, eps, ST);
+  const bool vec = cols % 4u == 0u && cols <= 8192u && ((uintptr_t)(X + c0) & 15u) == 0u && (ld % 4u == 0u || rows == 1u);
+  (vec ? k_rowstats<true> : k_rowstats<false>)<<<rows, 256, 0, st>>>(X, ld, c0, cols, mode, eps, ST);
   return cudaGetLastError();
 }
 
