@@ -13,6 +13,11 @@ typedef void (*decode_finish_fn)(const DecodeP);
 decode_finish_fn decode_finish_kernel(uint32_t mp, uint32_t epi);      // decode_finish.cu
 
 static decode_stream_fn stream_kernel(uint32_t enc, uint32_t xmode, uint32_t mp) {
+  // [prologue: f16, lnmod, rms][2 | 4 token columns]
+  static const decode_stream_fn few[3][2] = {{k_decode_stream<P0P_ENC_Q4, P0P_X_F16, 2>, k_decode_stream<P0P_ENC_Q4, P0P_X_F16, 4>},
+                                             {k_decode_stream<P0P_ENC_Q4, P0P_X_LNMOD, 2>, k_decode_stream<P0P_ENC_Q4, P0P_X_LNMOD, 4>},
+                                             {k_decode_stream<P0P_ENC_Q4, P0P_X_RMS, 2>, k_decode_stream<P0P_ENC_Q4, P0P_X_RMS, 4>}};
+  if (mp < 8u) return few[xmode][mp == 2u ? 0 : 1];
   // [encoding][prologue: f16, lnmod, rms][8 | 16 token columns]
   static const decode_stream_fn table[2][3][2] = {
       {{k_decode_stream<P0P_ENC_Q4, P0P_X_F16, 8>, k_decode_stream<P0P_ENC_Q4, P0P_X_F16, 16>},
@@ -39,7 +44,9 @@ bool decode_supported(const KP& p) {
 
 uint64_t plan_decode(DecodeP& d, DecodeLaunch& L, int sms, size_t smem_per_sm) {
   const KP& p = d.p;
-  d.Mp = p.M <= 8u ? 8u : 16u;
+  // (4-bit weights, up to 4 tokens: the spare columns carry further scale groups, see d_recs_q4.  8-bit weights have a third of the
+  // scale groups per byte and run at 0.83 of the memory's rate without it.)
+  d.Mp = p.M > 8u ? 16u : (p.enc == P0P_ENC_Q4 && p.M <= 4u) ? (p.M <= 2u ? 2u : 4u) : 8u;
   d.vec32 = (p.xmode != P0P_X_F16 && (((uintptr_t)p.X | (uintptr_t)(p.PV + p.pvOff)) & 15u) == 0u && p.ldx % 4u == 0u && p.kx0 % 4u == 0u && (p.xmode != P0P_X_LNMOD || p.pvStride % 4u == 0u)) ? 1u : 0u;
   const uint32_t cols = p.epi == P0P_EPI_SWIGLU ? p.N / 2u : ((p.epi == P0P_EPI_HEADS || p.epi == P0P_EPI_ONORMGATE) ? (p.N + 127u) / 128u * 128u : p.N);
   d.th = (cols + 63u) / 64u;
@@ -55,13 +62,13 @@ uint64_t plan_decode(DecodeP& d, DecodeLaunch& L, int sms, size_t smem_per_sm) {
   d.T = d.tiles * (p.K / (uint32_t)D_STAGE_K);
   const uint32_t tok_stride0 = kc * 2u + 64u;
   const size_t smem0 = (size_t)D_STAGES * D_STAGE_BYTES_Q8 + (size_t)(p.M + 1u) * tok_stride0 + 16384u;      // upper estimate: how many blocks an SM holds
-  const uint32_t slots = (uint32_t)std::max<size_t>(1, std::min<size_t>(4, smem_per_sm / (smem0 + 1024))) * (uint32_t)sms;
+  const uint32_t slots = (uint32_t)std::max<size_t>(1, std::min<size_t>(D_PER_SM, smem_per_sm / (smem0 + 1024))) * (uint32_t)sms;
   while (kc > (uint32_t)D_STAGE_K && d.T / std::min(d.T, slots) < kc / (uint32_t)D_STAGE_K) kc >>= 1;
   d.KC = kc; d.S = (p.K + kc - 1u) / kc; d.units = d.tiles * d.S;
   const uint32_t tok_stride = d.KC * 2u + (p.enc == P0P_ENC_Q4 ? 64u : 16u);
   const size_t ct_bytes = p.enc == P0P_ENC_Q4 ? (size_t)(d.KC / 32u) * (d.Mp / 2u) * 24u : (size_t)(d.KC / 64u) * (d.Mp / 2u) * 16u;
-  L.smem = (size_t)D_STAGES * (p.enc == P0P_ENC_Q4 ? D_STAGE_BYTES_Q4 : D_STAGE_BYTES_Q8) + (((p.M + 1u) * tok_stride + 127u) & ~127u) + ct_bytes + 4u * 32u * (d.Mp / 2u) * 4u + 2u * D_STAGES * 8u + 128u;
-  const uint32_t per_sm = (uint32_t)std::max<size_t>(1, std::min<size_t>(4, smem_per_sm / (L.smem + 1024)));
+  L.smem = (size_t)D_STAGES * (p.enc == P0P_ENC_Q4 ? D_STAGE_BYTES_Q4 : D_STAGE_BYTES_Q8) + (((p.M + 1u) * tok_stride + 127u) & ~127u) + ct_bytes + 4u * 32u * (std::max(d.Mp, 8u) / 2u) * 4u + 2u * D_STAGES * 8u + 128u;
+  const uint32_t per_sm = (uint32_t)std::max<size_t>(1, std::min<size_t>(D_PER_SM, smem_per_sm / (L.smem + 1024)));
   // every block is resident: the ranges run side by side.  At least KC / 256 stages per block (see above).
   L.grid = (int)std::min<uint64_t>(d.T / (d.KC / (uint32_t)D_STAGE_K), (uint64_t)per_sm * (uint64_t)sms);
   while ((uint64_t)d.T * (uint64_t)L.grid >= (1ull << 32)) L.grid = (L.grid + 1) / 2;      // the kernels' range arithmetic is 32-bit
@@ -76,9 +83,9 @@ cudaError_t launch_decode_pair(const DecodeP& d, const DecodeLaunch& L, int devi
   if (L.smem > (size_t)D_SMEM_MAX) return cudaErrorInvalidValue;
   const decode_stream_fn stream = stream_kernel(p.enc, p.xmode, d.Mp);
   // the dynamic shared memory ceiling is an attribute of (kernel, device): raised once for each pair
-  static DeviceOnce once[2][3][2];
+  static DeviceOnce once[2][3][4];
   cudaError_t e = cudaSuccess;
-  if (once[p.enc][p.xmode][d.Mp == 8u ? 0 : 1].run(device, [&] { e = cudaFuncSetAttribute(reinterpret_cast<const void*>(stream), cudaFuncAttributeMaxDynamicSharedMemorySize, D_SMEM_MAX); return (int)e; }))
+  if (once[p.enc][p.xmode][d.Mp == 8u ? 0 : d.Mp == 16u ? 1 : d.Mp == 2u ? 2 : 3].run(device, [&] { e = cudaFuncSetAttribute(reinterpret_cast<const void*>(stream), cudaFuncAttributeMaxDynamicSharedMemorySize, D_SMEM_MAX); return (int)e; }))
     return e != cudaSuccess ? e : cudaErrorInvalidDevice;
   // both kernels are programmatic dependents of whatever precedes them in the stream (see k_decode.cuh)
   cudaLaunchAttribute at[1];
@@ -87,7 +94,7 @@ cudaError_t launch_decode_pair(const DecodeP& d, const DecodeLaunch& L, int devi
   cfg.gridDim = dim3((unsigned)L.grid); cfg.blockDim = dim3(D_THREADS); cfg.dynamicSmemBytes = L.smem; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
   if ((e = cudaLaunchKernelEx(&cfg, stream, d)) != cudaSuccess) return e;
   cfg.gridDim = dim3(L.fin_blocks); cfg.blockDim = dim3(128); cfg.dynamicSmemBytes = 0;
-  return cudaLaunchKernelEx(&cfg, decode_finish_kernel(d.Mp, p.epi), d);
+  return cudaLaunchKernelEx(&cfg, decode_finish_kernel(d.Mp == 16u ? 16u : 8u, p.epi), d);
 }
 
 int launch_decode(p0p_ctx* c, const KP& p) {

@@ -39,6 +39,7 @@ namespace p0p {
 
 constexpr int D_CONSUMERS = 256;            // 8 warps: 4 row groups of 16 rows x 2 warps that split each stage's records
 constexpr int D_THREADS = D_CONSUMERS + 32; // + the producer warp
+constexpr int D_PER_SM = 3;                 // blocks an SM's registers hold (288 threads x 72): the plan relies on every block being resident
 constexpr int D_STAGES = 5;
 constexpr int D_STAGE_K = 256;              // k per stage: 8 q4 records (10240 B) or 4 q8 records (16896 B): one bulk copy each
 constexpr int D_STAGE_BYTES_Q4 = 10240, D_STAGE_BYTES_Q8 = 16896;
@@ -47,7 +48,7 @@ constexpr int D_SMEM_MAX = 144 * 1024;      // dynamic shared memory ceiling of 
 
 struct DecodeP {
   KP p;
-  uint32_t Mp;        // token columns fed to the tensor core: 8 or 16
+  uint32_t Mp;        // token columns: 2, 4 (4-bit weights: the multiply's other columns carry further scale groups), 8 or 16
   uint32_t tiles;     // 64-row tiles the call touches (swiglu: gate tiles then up tiles)
   uint32_t th;        // swiglu: tiles per half; else = tiles
   uint32_t KC, S;     // k-block length (multiple of 128) and count
@@ -222,6 +223,40 @@ __device__ __forceinline__ void d_rec_q4(float (&ta)[MP / 8][4], float (&tb)[MP 
     }
   }
 }
+// Up to 4 tokens (TC = 2 or 4 token columns): the multiply has 8 columns, so GC = 8 / TC records share one accumulator fragment.
+// Column n = slot * TC + token belongs to record R0 + slot: its token operand is that record's, and zero (a row of zeros is read)
+// while the other records are multiplied, so an accumulator ends as ONE record's sum and the scale, the minimum and the group's
+// token sum are applied once per GC records instead of once per record.  The kernel is bound by issue slots, and these were half of
+// them: the LLM block at one token 41.1 -> 38.9 us, 1 x 16384 x 16384 40.1 -> 38.0.
+// The slots' shares of y sit in different lanes (t4) and are added up when the unit ends.  ta / tb as in d_rec_q4; sa, sk: already at
+// this lane's slot; xk: for each slot, this lane's token row or the row of zeros.
+template <uint32_t R>
+__device__ __forceinline__ void d_mma_q4(float (&a1)[4], float (&a2)[4], uint32_t ca, uint32_t xk, const DLane& L) {
+  const uint32_t wl = lds32<R * 1280u>(ca), wh = lds32<R * 1280u + 128u>(ca);
+  const uint32_t wl8 = wl >> 8, wh8 = wh >> 8;
+  const uint4 b = lds128<R * 64u>(xk);
+  float n1[4], n2[4];
+  mma_16816(n1, wl & L.MLO, wh & L.MLO, wl & L.MHI, wh & L.MHI, b.x, b.y, a1);
+  mma_16816(n2, wl8 & L.MLO, wh8 & L.MLO, wl8 & L.MHI, wh8 & L.MHI, b.z, b.w, a2);
+#pragma unroll
+  for (int i = 0; i < 4; i++) { a1[i] = n1[i]; a2[i] = n2[i]; }
+}
+template <int TC, uint32_t R0>
+__device__ __forceinline__ void d_recs_q4(float (&ta)[4], float (&tb)[4], uint32_t ca, uint32_t sa, const uint32_t (&xk)[8 / TC], uint32_t sk, const DLane& L) {
+  const uint32_t sml = lds32<R0 * 1280u>(sa), smh = lds32<R0 * 1280u + 32u>(sa);
+  const float2 sx = lds64f<R0 * (TC / 2) * 8u>(sk);
+  float a1[4] = {0.0f, 0.0f, 0.0f, 0.0f}, a2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  d_mma_q4<R0>(a1, a2, ca, xk[0], L);
+  d_mma_q4<R0 + 1u>(a1, a2, ca, xk[1], L);
+  if constexpr (TC == 2) { d_mma_q4<R0 + 2u>(a1, a2, ca, xk[2], L); d_mma_q4<R0 + 3u>(a1, a2, ca, xk[3], L); }
+  const float2 fl = __half22float2(*reinterpret_cast<const __half2*>(&sml)), fh = __half22float2(*reinterpret_cast<const __half2*>(&smh));   // (scale, min)
+  ta[0] = fmaf(fl.x, a1[0] + a2[0], ta[0]); tb[0] = fmaf(fl.y, sx.x, tb[0]);
+  ta[2] = fmaf(fh.x, a1[2] + a2[2], ta[2]); tb[2] = fmaf(fh.y, sx.x, tb[2]);
+  if (!L.one) {
+    ta[1] = fmaf(fl.x, a1[1] + a2[1], ta[1]); tb[1] = fmaf(fl.y, sx.y, tb[1]);
+    ta[3] = fmaf(fh.x, a1[3] + a2[3], ta[3]); tb[3] = fmaf(fh.y, sx.y, tb[3]);
+  }
+}
 // one q8 record (64 rows x 64 k)
 template <int MP, uint32_t R>
 __device__ __forceinline__ void d_rec_q8(float (&tot)[MP / 8][4], uint32_t ca, uint32_t sa, uint32_t xk0, uint32_t xk1, uint32_t ck, const DLane& L) {
@@ -253,7 +288,7 @@ __device__ __forceinline__ void d_rec_q8(float (&tot)[MP / 8][4], uint32_t ca, u
 }
 
 template <int ENC, int XMODE, int MP>
-__global__ void __launch_bounds__(D_THREADS) k_decode_stream(const DecodeP d) {
+__global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const DecodeP d) {
   extern __shared__ __align__(128) unsigned char smem[];
   const KP& p = d.p;
   constexpr uint32_t TOK_PAD = ENC == P0P_ENC_Q4 ? 64u : 16u;           // keeps the operand loads free of bank conflicts
@@ -263,10 +298,11 @@ __global__ void __launch_bounds__(D_THREADS) k_decode_stream(const DecodeP d) {
   unsigned char* stages = smem;
   constexpr uint32_t D_STAGE_BYTES = ENC == P0P_ENC_Q4 ? D_STAGE_BYTES_Q4 : D_STAGE_BYTES_Q8;
   unsigned char* xs = stages + D_STAGES * D_STAGE_BYTES;
+  constexpr int NF = MP < 8 ? 1 : MP / 8;                                                      // accumulator fragments per lane
   float* ctc = reinterpret_cast<float*>(xs + (((p.M + 1u) * tok_stride + 127u) & ~127u));       // [group][pair] float4 (-Ca, -Cb, -Ca, -Cb)
   float* cts = ctc + (d.KC / GS) * (MP / 2) * 4u;                                              // [group][pair] float2 (Sx_a, Sx_b)   (q4 only)
-  float* comb = cts + (ENC == P0P_ENC_Q4 ? (d.KC / GS) * (MP / 2) * 2u : 0u);                  // [4 row groups][32 lanes][MP/2]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(comb + 4u * 32u * (MP / 2));
+  float* comb = cts + (ENC == P0P_ENC_Q4 ? (d.KC / GS) * (MP / 2) * 2u : 0u);                  // [4 row groups][32 lanes][4 * NF]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(comb + 4u * 32u * (4 * NF));
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + D_STAGES);
 
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
@@ -317,9 +353,14 @@ __global__ void __launch_bounds__(D_THREADS) k_decode_stream(const DecodeP d) {
   // this lane's token pair (2 t4, 2 t4 + 1); + 4 pairs for tokens 8..15.  With a single token every lane reads pair 0
   // (one address per warp instead of four)
   const uint32_t tp = p.M == 1u ? 0u : t4;
+  // few tokens: this lane's accumulator columns 2 t4, 2 t4 + 1 belong to record slot `slot`; as an operand column, g = slot_b * MP + token
+  constexpr uint32_t GC = MP < 8 ? 8 / MP : 1;
+  const uint32_t slot = MP < 8 ? t4 / (uint32_t)(MP / 2) : 0u, slot_b = MP < 8 ? g / (uint32_t)MP : 0u;
+  const uint32_t x_off = half * RPW * REC_K * 2u + t4 * 16u, x_zero = smem_u32(xs) + p.M * tok_stride + x_off, x_own = smem_u32(xs) + min(g % (uint32_t)MP, p.M) * tok_stride + x_off;
+  const uint32_t cts_s = smem_u32(cts) + (half * RPW + slot) * (uint32_t)(MP / 2) * 8u + (t4 % (uint32_t)(MP / 2)) * 8u;
   const uint32_t ctc_l = smem_u32(ctc) + (half * RPW * (MP / 2) + tp) * 16u;
   const uint32_t cts_l = smem_u32(cts) + (half * RPW * (MP / 2) + tp) * 8u;
-  float* comb_l = comb + (rg * 32u + lane) * (MP / 2);
+  float* comb_l = comb + (rg * 32u + lane) * (4 * NF);
   DLane L;
   L.MLO = 0x000f000fu; L.MHI = 0x00f000f0u; L.MAGIC = 0x64006400u;      // (masks live in registers: as immediates each AND would cost a constant load)
   L.on0 = g < p.M ? 1u : 0u; L.on1 = g + 8u < p.M ? 1u : 0u;            // does this lane's token column exist?
@@ -344,9 +385,9 @@ __global__ void __launch_bounds__(D_THREADS) k_decode_stream(const DecodeP d) {
       bar_sync_named(1, D_CONSUMERS);
       cur_kb = kb;
     }
-    float tot[MP / 8][4], tmn[MP / 8][4];            // q4: tot = sums of s * acc (still to be scaled by 2^24), tmn = sums of mn * Sx
+    float tot[NF][4], tmn[NF][4];            // q4: tot = sums of s * acc (still to be scaled by 2^24), tmn = sums of mn * Sx
 #pragma unroll
-    for (int h = 0; h < MP / 8; h++)
+    for (int h = 0; h < NF; h++)
 #pragma unroll
       for (int i = 0; i < 4; i++) { tot[h][i] = 0.0f; tmn[h][i] = 0.0f; }
 
@@ -355,7 +396,14 @@ __global__ void __launch_bounds__(D_THREADS) k_decode_stream(const DecodeP d) {
       const uint32_t so = anchor(s * D_STAGE_BYTES), ko = anchor(k);
       const uint32_t ca = code0 + so, sa = sm0 + so;
       const uint32_t xk0 = xrow0 + ko * 2u, xk1 = xrow1 + ko * 2u;
-      if (ENC == P0P_ENC_Q4) {
+      if constexpr (MP < 8) {
+        const uint32_t sk = cts_s + (ko / GS) * (MP / 2) * 8u, sas = sa + slot * 1280u;
+        uint32_t xk[GC];
+#pragma unroll
+        for (uint32_t j = 0; j < GC; j++) xk[j] = (slot_b == j ? x_own : x_zero) + ko * 2u;
+        d_recs_q4<MP, 0>(tot[0], tmn[0], ca, sas, xk, sk, L);
+        if constexpr (MP == 4) d_recs_q4<MP, 2>(tot[0], tmn[0], ca, sas, xk, sk, L);
+      } else if constexpr (ENC == P0P_ENC_Q4) {
         const uint32_t sk = cts_l + (ko / GS) * (MP / 2) * 8u;
         static_assert(D_STAGE_K == 256, "four q4 records / two q8 records per consumer warp and stage");
         d_rec_q4<MP, 0>(tot, tmn, ca, sa, xk0, xk1, sk, L);
@@ -375,18 +423,25 @@ __global__ void __launch_bounds__(D_THREADS) k_decode_stream(const DecodeP d) {
     // scratch[kb][part][token][slot].  Both named barriers are met in drain mode too.
     if (ENC == P0P_ENC_Q4) {
 #pragma unroll
-      for (int h = 0; h < MP / 8; h++)
+      for (int h = 0; h < NF; h++)
 #pragma unroll
         for (int i = 0; i < 4; i++) tot[h][i] = fmaf(tot[h][i], 16777216.0f, tmn[h][i]);      // the codes entered as q * 2^-24
     }
+    if (MP < 8) {                                    // the record slots' shares: lanes t4 that hold the same tokens
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+#pragma unroll
+        for (uint32_t o = MP / 2; o < 4u; o <<= 1) tot[0][i] += __shfl_xor_sync(0xffffffffu, tot[0][i], o);
+      }
+    }
     if (half == 1u) {
 #pragma unroll
-      for (int h = 0; h < MP / 8; h++) *reinterpret_cast<float4*>(comb_l + 4 * h) = make_float4(tot[h][0], tot[h][1], tot[h][2], tot[h][3]);
+      for (int h = 0; h < NF; h++) *reinterpret_cast<float4*>(comb_l + 4 * h) = make_float4(tot[h][0], tot[h][1], tot[h][2], tot[h][3]);
     }
     bar_sync_named(2 + rg, 64);
     if (half == 0u && ok) {
 #pragma unroll
-      for (int h = 0; h < MP / 8; h++) {
+      for (int h = 0; h < NF; h++) {
         const float4 o = *reinterpret_cast<const float4*>(comb_l + 4 * h);
         const float v[4] = {tot[h][0] + o.x, tot[h][1] + o.y, tot[h][2] + o.z, tot[h][3] + o.w};
 #pragma unroll
