@@ -56,7 +56,6 @@ struct UmmaP {
   KP p;
   uint32_t BT;          // tokens per tile: a multiple of 16 up to 256 (one UMMA of N = BT), or of 32 up to 384 (two of N = BT / 2)
   uint32_t NACC;        // accumulators: 2 (the next tile's multiply overlaps the epilogue) or 1 (wide tiles: tensor memory holds one)
-  uint32_t KSPLIT;      // accumulators per tile that take the 16-k multiplies in turn (1, 2 or 4), summed by the epilogue
   uint32_t NS;          // stages of the token ring (2 .. 8)
   uint32_t KW;          // k-steps of 64 k per pipeline step (1, 2 or 4)
   uint32_t NA;          // stages of the dequantised operand in tensor memory (a_col0 + NA * KW * 32 <= 512, NA <= 8); fp16 weights: = NS
@@ -64,13 +63,15 @@ struct UmmaP {
   uint32_t a_col0;      // first tensor-memory column of the operand stages (quantised weights): the accumulators end there
   uint32_t LOCK;        // 1: the token ring and the operand ring advance together and share their barriers (NA == NS)
   uint32_t NQ;          // stages of quantised records (each KSUP k-steps long)
-  uint32_t n_tiles, m_tiles;
+  uint32_t n_tiles, m_tiles;   // n_tiles: of 128 columns, or with PAIR of 256 (two blocks of 128 columns each)
+  uint32_t PAIR;        // 1: two blocks (a cluster, one SM each) work on one tile of 256 columns
+  uint32_t nt_all;      // 128-column tiles there are (odd: the last pair's second block computes columns that are not stored)
   uint32_t G;           // token tiles per group of the tile order (tile_coords)
   uint32_t cvR;         // conv3: image rows per token tile (tile = cvR x Wo output positions of one frame)
   uint32_t T0, S, ks_per;   // split-K: the first T0 tiles (in tile order) are whole units; each of the rest is S units of ks_per
                             // k-steps whose fp32 partial sums go to sk_part.  T0 = all tiles: no split; T0 = 0: every tile split;
                             // in between: only the tiles of the last, nearly empty round are split over the idle SMs
-  float* sk_part;           // [S][tiles - T0][BT][128] partial sums (k_umma_finish adds them and applies the epilogue)
+  float* sk_part;           // [S][tiles - T0][1 or 2 blocks][BT][128] partial sums (k_umma_finish adds them and applies the epilogue)
   int* status;
 };
 
@@ -145,20 +146,36 @@ constexpr uint32_t U_NX_MAX = 8;         // most stages of the token ring
 // parked by the hardware (mbar_try), not spinning beside the ones that work.
 // KW and LOCK are compile-time (four variants exist: (1, lock), (2, lock), (2, separate), (4, separate; 4-bit weights)): the issuing warp's loop is the
 // critical path of wide tiles and must not carry run-time choices.
-template <int ENC, int EPI, int KW_, bool LOCK_>
+//
+// PAIR: two blocks of a cluster (the two SMs of a TPC) compute one tile of 256 columns x BT tokens with tcgen05's cta_group::2.
+// Each block holds 128 weight rows - its own operand ring and accumulator, as without PAIR - but only HALF of the token tile: a
+// multiply reads the tokens from both blocks' shared memory.  Above 128 tokens a lone block is bound by its shared memory (a
+// 128-k step of 256 tokens: 64 KB written by TMA, 64 KB read by the multiplies, 20 KB of records written and read, at 128 B per
+// clock: over 1150 cycles against 912 for the multiplies); a pair moves half the tokens per SM, and twice as many stages fit.  Block 0
+// of the pair issues the multiplies: its operand barriers collect the arrivals of both blocks (the dequantisation warps arrive
+// across the cluster, the token loads of block 1 complete on block 0's barrier), and its commits arrive in both.  These arrivals
+// have no cluster scope of their own (with .release.cluster every hand-over paid a memory barrier: 41 us against 25 at q8,
+// 130 x 14336 x 4096): what they publish lies in tensor memory and is ordered by the tcgen05 fences around them.  The rule that
+// picks pairs, and what both sides measured, stands in launch_umma.
+template <int ENC, int EPI, int KW_, bool LOCK_, bool PAIR = false>
 __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const __grid_constant__ CUtensorMap mapX, const __grid_constant__ CUtensorMap mapW) {
   extern __shared__ unsigned char smem_raw[];
   constexpr bool ATM = ENC != P0P_ENC_F16;
   constexpr uint32_t KW = KW_;
   using Q = UQ<ENC, KW_>;
   constexpr bool lock = LOCK_;
+  constexpr int CG = PAIR ? 2 : 1;
+  constexpr uint32_t NB = PAIR ? 2u : 1u;                                          // blocks per tile
+  static_assert(!PAIR || LOCK_, "a pair's token and operand rings share their barriers");
+  const uint32_t rank = PAIR ? cluster_rank() : 0u, bid = blockIdx.x / NB, nblk = gridDim.x / NB;
   const KP& p = u.p;
   const uint32_t BT = u.BT, NS = u.NS, NQ = u.NQ;
   const uint32_t HB = BT > 256u ? BT / 2u : BT, NH = BT > 256u ? 2u : 1u;          // tokens per UMMA / TMA box, and how many of them make a tile
   const bool two_acc = u.NACC == 2u;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;                     // operand tiles need 1024-byte alignment
   unsigned char* gbase = smem_raw + (base - smem_u32(smem_raw));
-  const uint32_t XT = BT * 128u, XS = KW * XT;                                     // bytes of a token sub-tile (64 k) and of a stage
+  const uint32_t HR = HB / NB;                                                     // ... of which this block's shared memory holds HR
+  const uint32_t XT = NH * HR * 128u, XS = KW * XT;                                     // bytes of a token sub-tile (64 k) and of a stage
   const uint32_t a_st = base, x_st = a_st + (ATM ? 0u : NS * U_A_BYTES), q_st = x_st + NS * XS;
   const uint32_t acc_stride = u.acc_stride;
   const uint32_t epi_sh = q_st + (ENC == P0P_ENC_F16 ? 0u : NQ * Q::STAGE);
@@ -168,6 +185,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
   const uint32_t xfull = bars, xempty = xfull + 8u * U_NX_MAX, afull = xempty + 8u * U_NX_MAX, aempty = afull + 8u * U_NA_MAX;
   const uint32_t wq_full = aempty + 8u * U_NA_MAX, wq_empty = wq_full + 8u * U_NQ_MAX;
   const uint32_t acc_full = wq_empty + 8u * U_NQ_MAX, acc_empty = acc_full + 16u, tmem_slot = acc_empty + 16u;
+  constexpr bool ALT = KW == 1u || !lock || PAIR;                                // how the two dequantisation groups share the steps (see there)
   const uint32_t NA = u.NA;                                                       // operand stage of step g: g % NA, its parity: (g / NA) & 1
   const uint32_t pfull = lock ? afull : xfull, pempty = lock ? aempty : xempty;   // the barriers the token producer works with
 
@@ -178,14 +196,14 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
   const uint32_t tid = threadIdx.x, warp = __shfl_sync(0xffffffffu, tid >> 5, 0), lane = tid & 31u;
   if (tid == 0) {
     for (uint32_t s = 0; s < U_NX_MAX; s++) { mbar_init(xfull + 8u * s, 1u); mbar_init(xempty + 8u * s, 1u); }      // the producer's expect_tx arrival / the multiplies' commit
-    for (uint32_t s = 0; s < U_NA_MAX; s++) { mbar_init(afull + 8u * s, (ATM ? (KW == 2u && lock ? 8u : 4u) : 0u) + (lock ? 1u : 0u)); mbar_init(aempty + 8u * s, 1u); }       // the dequantisation warps of a step (+ the token producer) / the commit
+    for (uint32_t s = 0; s < U_NA_MAX; s++) { mbar_init(afull + 8u * s, (ATM ? NB * (ALT ? 4u : 8u) : 0u) + (lock ? 1u : 0u)); mbar_init(aempty + 8u * s, 1u); }       // the dequantisation warps of a step (+ the token producer) / the commit
     for (uint32_t s = 0; s < (uint32_t)U_NQ_MAX; s++) { mbar_init(wq_full + 8u * s, 1u); mbar_init(wq_empty + 8u * s, U_DEQ_WARPS); }
-    for (uint32_t b = 0; b < 2u; b++) { mbar_init(acc_full + 8u * b, 1u); mbar_init(acc_empty + 8u * b, 4u); }
+    for (uint32_t b = 0; b < 2u; b++) { mbar_init(acc_full + 8u * b, 1u); mbar_init(acc_empty + 8u * b, NB * 4u); }
     fence_mbar_init();
   }
-  if (warp == 1) { tmem_alloc(tmem_slot, U_TMEM_COLS); tmem_relinquish(); }
+  if (warp == 1) { tmem_alloc<CG>(tmem_slot, U_TMEM_COLS); tmem_relinquish<CG>(); }
   tc_fence_before();
-  __syncthreads();
+  if (PAIR) cluster_sync(); else __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base)), 0);
 
@@ -197,14 +215,17 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     if (lane == 0) {
       Ring r(NS);
       bool ok = true;
+      auto load2 = [&](uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar) { if (PAIR) tma_load_2d_pair(dst, m, x, y, bar); else tma_load_2d(dst, m, x, y, bar); };
+      auto load4 = [&](uint32_t dst, int c0, int c1, int c2, int c3, uint32_t bar) { if (PAIR) tma_load_4d_pair(dst, &mapX, c0, c1, c2, c3, bar); else tma_load_4d(dst, &mapX, c0, c1, c2, c3, bar); };
       const uint32_t nap = BT <= 64u ? 32u : 200u;                     // narrow tiles turn over quickly: poll their stages often
-      for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+      for (uint32_t unit = bid; unit < units && ok; unit += nblk) {
         const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t tile = un.tile, kb = un.kb, ke = un.ke;
-        uint32_t nt, mt; tile_coords(u, tile, nt, mt);
+        uint32_t nt, mt; tile_coords(u, tile, nt, mt); nt = nt * NB + rank;
         for (uint32_t k0 = kb; k0 < ke; k0 += KW, r.next()) {
           const uint32_t cnt = min(KW, ke - k0);
           if (!mbar_wait(pempty + 8u * r.s, r.ph ^ 1u, u.status, 201, nap)) { ok = false; break; }
-          mbar_expect_tx(pfull + 8u * r.s, cnt * (XT + (ENC == P0P_ENC_F16 ? U_A_BYTES : 0u)));
+          if (rank == 0u) mbar_expect_tx(pfull + 8u * r.s, NB * cnt * (XT + (ENC == P0P_ENC_F16 ? U_A_BYTES : 0u)));      // (both blocks' loads complete on block 0's barrier)
+          const uint32_t fb = PAIR ? cluster_addr(pfull + 8u * r.s, 0u) : pfull + 8u * r.s;
           for (uint32_t j = 0; j < cnt; j++) {
             const uint32_t ks = k0 + j, dst = x_st + r.s * XS + j * XT;
             if (p.xmode == P0P_X_CONV3) {
@@ -217,7 +238,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
               const int it = p.ks > 1u ? itg % (int)p.ks : itg - (int)p.padL;
               const uint32_t rb = u.cvR / NH;
               for (uint32_t h = 0; h < NH; h++)
-                tma_load_4d(dst + h * HB * 128u, &mapX, (int)c0, (int)kx - 1, (int)(oy0 + h * rb + ky) - 1, it, pfull + 8u * r.s);
+                load4(dst + h * HR * 128u, (int)c0, (int)kx - 1, (int)(oy0 + h * rb + rank * (rb / NB) + ky) - 1, it, fb);
             } else if (p.xmode == P0P_X_CONV) {
               // 2-D implicit GEMM (src/ops/gemm.js:81-91): the tile's tokens are cvR whole output rows; the 64 k of this k-step are
               // channels c0.. of one tap (ky, kx) = (tap / ks, tap % ks).  The tensor map's element strides walk the input by the
@@ -227,10 +248,10 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
               const uint32_t kg = ks * 64u, tap = kg / p.Ci, c0 = kg - tap * p.Ci, ky = tap / p.ks, kx = tap - ky * p.ks;
               const uint32_t rb = u.cvR / NH;
               for (uint32_t h = 0; h < NH; h++)
-                tma_load_4d(dst + h * HB * 128u, &mapX, (int)c0, (int)kx - (int)p.padL, (int)((oy0 + h * rb) * p.stride + ky) - (int)p.padT, 0, pfull + 8u * r.s);
+                load4(dst + h * HR * 128u, (int)c0, (int)kx - (int)p.padL, (int)((oy0 + h * rb + rank * (rb / NB)) * p.stride + ky) - (int)p.padT, 0, fb);
             } else
-              for (uint32_t h = 0; h < NH; h++) tma_load_2d(dst + h * HB * 128u, &mapX, (int)(ks * 64u), (int)(mt * BT + h * HB), pfull + 8u * r.s);
-            if (ENC == P0P_ENC_F16) tma_load_2d(a_st + (r.s * KW + j) * U_A_BYTES, &mapW, (int)(ks * 64u), (int)(p.wR0 + nt * 128u), pfull + 8u * r.s);
+              for (uint32_t h = 0; h < NH; h++) load2(dst + h * HR * 128u, &mapX, (int)(ks * 64u), (int)(mt * BT + h * HB + rank * HR), fb);
+            if (ENC == P0P_ENC_F16) load2(a_st + (r.s * KW + j) * U_A_BYTES, &mapW, (int)(ks * 64u), (int)(p.wR0 + nt * 128u), fb);
           }
         }
       }
@@ -242,9 +263,9 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
       Ring q(NQ);
       bool ok = true;
       const uint32_t last = (p.Nw >> 6) - 1u;                  // record tiles past the weight's end do not exist: their columns are never stored
-      for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+      for (uint32_t unit = bid; unit < units && ok; unit += nblk) {
         const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t tile = un.tile, kb = un.kb, ke = un.ke;
-        uint32_t nt, mt; tile_coords(u, tile, nt, mt);
+        uint32_t nt, mt; tile_coords(u, tile, nt, mt); nt = nt * NB + rank;
         uint32_t trow[2];
         if (swiglu) { trow[0] = min((p.wR0 + nt * 64u) >> 6, last); trow[1] = min((p.wR1 + nt * 64u) >> 6, last); }
         else { trow[0] = min((p.wR0 + nt * 128u) >> 6, last); trow[1] = min(trow[0] + 1u, last); }
@@ -260,24 +281,26 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
       }
     }
   } else if (warp == 1) {
+   if (rank == 0u) {
     // ================================================================= MMA issuer.  The WHOLE warp walks the loop and one
     // elected lane issues: in warp-uniform control flow the descriptors live in uniform registers, which is what the
     // instruction takes; inside a one-lane branch every operand of every tcgen05.mma is first moved there, which
     // costs more than the multiply itself.
-    const uint32_t idesc = umma_idesc_f16(128u, HB);
+    const uint32_t idesc = umma_idesc_f16(128u * NB, HB);
+    auto wait_op = [&](uint32_t bar, uint32_t par, int code, uint32_t ns = 0u) { return mbar_wait(bar, par, u.status, code, ns); };
     Ring r(NS), ar(NA);
     uint32_t tl = 0;
     bool ok = true;
-    for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x, tl++) {
+    for (uint32_t unit = bid; unit < units && ok; unit += nblk, tl++) {
       const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t kb = un.kb, ke = un.ke;
       const uint32_t buf = two_acc ? tl & 1u : 0u, par = two_acc ? (tl >> 1) & 1u : tl & 1u;
-      if (!__all_sync(0xffffffffu, mbar_wait(acc_empty + 8u * buf, par ^ 1u, u.status, 203, 100u))) { ok = false; break; }
+      if (!__all_sync(0xffffffffu, wait_op(acc_empty + 8u * buf, par ^ 1u, 203, 100u))) { ok = false; break; }
       tc_fence_after();
       const uint32_t d_tmem = tmem_base + buf * acc_stride;
       for (uint32_t k0 = kb; k0 < ke; k0 += KW, r.next(), ar.next()) {
         const uint32_t as = ar.s, cnt = min(KW, ke - k0);
-        bool rdy = lock || mbar_wait(xfull + 8u * r.s, r.ph, u.status, 204);
-        if (ATM || lock) rdy = rdy && mbar_wait(afull + 8u * as, ar.ph, u.status, 205);
+        bool rdy = lock || wait_op(xfull + 8u * r.s, r.ph, 204);
+        if (ATM || lock) rdy = rdy && wait_op(afull + 8u * as, ar.ph, 205);
         if (!__all_sync(0xffffffffu, rdy)) { ok = false; break; }
         tc_fence_after();
         // (operands computed in warp-uniform control flow: they stay in uniform registers, which is what the instruction takes)
@@ -295,36 +318,36 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
             if (j < cnt) {
 #pragma unroll
               for (uint32_t kk = 0; kk < 4u; kk++) {                  // per 16 k: 8 tensor-memory columns / +32 bytes
-                // consecutive multiplies into ONE accumulator start ~180 cycles apart whatever their width; into different
-                // accumulators ~35.  Narrow tiles therefore rotate over KSPLIT accumulators (wide ones over their two halves).
-                const uint32_t dk = d_tmem + (kk & (u.KSPLIT - 1u)) * BT, accum = first | j | (kk >= u.KSPLIT ? 1u : 0u);
+                const uint32_t accum = first | j | kk;
                 if (ATM) {
-                  umma_f16_ts(dk, at[j] + 8u * kk, bd[j] + 2u * kk, idesc, accum);
-                  if (NH == 2u) umma_f16_ts(dk + HB, at[j] + 8u * kk, bd[j] + ((HB * 128u) >> 4) + 2u * kk, idesc, accum);
+                  umma_f16_ts<CG>(d_tmem, at[j] + 8u * kk, bd[j] + 2u * kk, idesc, accum);
+                  if (NH == 2u) umma_f16_ts<CG>(d_tmem + HB, at[j] + 8u * kk, bd[j] + ((HR * 128u) >> 4) + 2u * kk, idesc, accum);
                 } else {
-                  umma_f16_ss(dk, ad[j] + 2u * kk, bd[j] + 2u * kk, idesc, accum);
-                  if (NH == 2u) umma_f16_ss(dk + HB, ad[j] + 2u * kk, bd[j] + ((HB * 128u) >> 4) + 2u * kk, idesc, accum);
+                  umma_f16_ss<CG>(d_tmem, ad[j] + 2u * kk, bd[j] + 2u * kk, idesc, accum);
+                  if (NH == 2u) umma_f16_ss<CG>(d_tmem + HB, ad[j] + 2u * kk, bd[j] + ((HR * 128u) >> 4) + 2u * kk, idesc, accum);
                 }
               }
             }
           }
-          if (!lock) umma_commit(xempty + 8u * r.s);
-          if (ATM || lock) umma_commit(aempty + 8u * as);
+          if (!lock) umma_commit<CG>(xempty + 8u * r.s);
+          if (ATM || lock) umma_commit<CG>(aempty + 8u * as);
         }
         __syncwarp();
       }
-      if (ok && elect_one()) umma_commit(acc_full + 8u * buf);
+      if (ok && elect_one()) umma_commit<CG>(acc_full + 8u * buf);
       __syncwarp();
     }
+   }
   } else if (warp < 6) {
     // ================================================================= epilogue (TMEM lanes 32*(warp%4) .. +31)
     const uint32_t q = warp & 3u, c = q * 32u + lane;
     uint32_t tl = 0, pass = 0;
     bool ok = true;
     const bool vec = epilogue_vec_ok(p);
-    for (uint32_t unit = blockIdx.x; unit < units; unit += gridDim.x, tl++) {
+    auto acc_free = [&](uint32_t b) { if (PAIR) mbar_arrive_cluster(cluster_addr(acc_empty + 8u * b, 0u)); else mbar_arrive(acc_empty + 8u * b); };
+    for (uint32_t unit = bid; unit < units; unit += nblk, tl++) {
       const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t tile = un.tile, sp = un.sp;
-      uint32_t nt, mt; tile_coords(u, tile, nt, mt);
+      uint32_t nt, mt; tile_coords(u, tile, nt, mt); nt = nt * NB + rank;
       const uint32_t buf = two_acc ? tl & 1u : 0u, par = two_acc ? (tl >> 1) & 1u : tl & 1u;
       if (ok && !mbar_wait(acc_full + 8u * buf, par, u.status, 206, 1000u)) ok = false;
       tc_fence_after();
@@ -337,20 +360,16 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
         tmem_ld_wait();
 #pragma unroll
         for (int j = 0; j < U_EPI_TB; j++) acc[j] = ok ? __uint_as_float(r[j]) : 0.0f;
-        for (uint32_t a = 1; a < u.KSPLIT; a++) {            // the tile's other accumulators (narrow tiles only: few passes)
-          tmem_ld16(t0 + a * BT + ch * U_EPI_TB, r); tmem_ld_wait();
-#pragma unroll
-          for (int j = 0; j < U_EPI_TB; j++) acc[j] += ok ? __uint_as_float(r[j]) : 0.0f;
-        }
         if (ch + 1u < nchunks) tmem_ld16(t0 + (ch + 1u) * U_EPI_TB, r);      // the next pass's accumulators load behind this pass's work
         else {                                                   // the tile's last values are in registers: the accumulator is free for
           tc_fence_before();                                     // the next tile's multiplies while this pass still computes and stores
           __syncwarp();
-          if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
+          if (lane == 0) acc_free(buf);
         }
+        if (PAIR && nt >= u.nt_all) continue;                    // (the missing last tile of an odd count: uniform over the four warps)
         if (un.split) {
           // split-K: this unit's partial sums, fp32, to its own slab; a warp's store covers 128 bytes of a row
-          float* dst = u.sk_part + (((size_t)sp * (tiles - u.T0) + (tile - u.T0)) * BT + ch * U_EPI_TB) * 128u + c;
+          float* dst = u.sk_part + ((((size_t)sp * (tiles - u.T0) + (tile - u.T0)) * NB + rank) * BT + ch * U_EPI_TB) * 128u + c;
 #pragma unroll
           for (int j = 0; j < U_EPI_TB; j++) dst[(size_t)j * 128u] = acc[j];
         } else epilogue_cols<U_EPI_TB, EPI>(p, m0 + ch * U_EPI_TB, nt * 128u, c, acc, epi_ptr, 2, vec, pass & 1u);
@@ -358,7 +377,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
       if (nchunks == 0u) {                                       // (cannot happen: a tile has tokens; kept so that the barrier's count never slips)
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(acc_empty + 8u * buf);
+        if (lane == 0) acc_free(buf);
       }
     }
   } else if (ENC != P0P_ENC_F16 && warp < 6u + U_DEQ_WARPS) {
@@ -377,7 +396,6 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     // take whole steps in turn, so a warp pays its trip round this loop - a few hundred cycles of serial latency whatever the work -
     // once per step it converts, and with three or more operand stages neither group waits for the multiplies of its own last
     // step.  Steps of 128 k in lock step (two stages only): group g converts sub-step g of every step, both side by side.
-    constexpr bool ALT = KW == 1u || !lock;
     const uint32_t stride = ALT ? 2u : 1u;
     uint32_t as = ALT ? grp : 0u, aph = 0u;
     Ring qr(NQ);
@@ -408,7 +426,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
         }
       }
     };
-    for (uint32_t unit = blockIdx.x; unit < units && ok; unit += gridDim.x) {
+    for (uint32_t unit = bid; unit < units && ok; unit += nblk) {
       const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t n = un.ke - un.kb;
       for (uint32_t j0 = 0; j0 < n && ok; j0 += Q::KSUP, qr.next()) {
         const uint32_t cnt = min(Q::KSUP, n - j0);
@@ -424,7 +442,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
               if (st * KW + sub < cnt) convert(st * KW + sub, ta0 + (as * KW + sub) * 32u);
             tmem_st_wait(); tc_fence_before();                      // tensor-memory stores done and ordered before the MMA warp's read
             __syncwarp();
-            if (lane == 0) mbar_arrive(afull + 8u * as);
+            if (lane == 0) { if (PAIR) mbar_arrive_cluster(cluster_addr(afull + 8u * as, 0u)); else mbar_arrive(afull + 8u * as); }
             as += stride; if (as >= NA) { as -= NA; aph ^= 1u; }
           }
           gpar ^= nst & 1u;
@@ -454,10 +472,10 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
       }
     }
   }
-  // ---- wind down: every role is past its last use of tensor memory
+  // ---- wind down: every role is past its last use of tensor memory (and, in a pair, of the other block's barriers)
   tc_fence_before();
-  __syncthreads();
-  if (warp == 1) { tc_fence_after(); tmem_dealloc(tmem_base, U_TMEM_COLS); }
+  if (PAIR) cluster_sync(); else __syncthreads();
+  if (warp == 1) { tc_fence_after(); tmem_dealloc<CG>(tmem_base, U_TMEM_COLS); }
 }
 
 // ---- split-K second stage: the S partial sums of 16 tokens x 128 columns of a split tile are added in split order
@@ -466,10 +484,11 @@ template <int EPI>
 __global__ void __launch_bounds__(128) k_umma_finish(const UmmaP u) {
   __shared__ __align__(16) float sh[2 * U_EPI_TB * 132];
   const KP& p = u.p;
-  const uint32_t tiles = u.n_tiles * u.m_tiles, tail = tiles - u.T0, t = blockIdx.x, c = threadIdx.x;
-  uint32_t nt, mt; tile_coords(u, u.T0 + t, nt, mt);
+  const uint32_t tiles = u.n_tiles * u.m_tiles, NB = 1u + u.PAIR, tail = (tiles - u.T0) * NB, t = blockIdx.x, c = threadIdx.x;      // (slots of 128 columns: NB per tile)
+  uint32_t nt, mt; tile_coords(u, u.T0 + t / NB, nt, mt);
+  nt = nt * NB + t % NB;
   const uint32_t r0 = blockIdx.y * U_EPI_TB, m0 = mt * u.BT + r0;
-  if (m0 >= p.M) return;
+  if (m0 >= p.M || nt >= u.nt_all) return;
   float acc[U_EPI_TB];
 #pragma unroll
   for (int j = 0; j < U_EPI_TB; j++) acc[j] = 0.0f;
@@ -485,15 +504,16 @@ __global__ void __launch_bounds__(128) k_umma_finish(const UmmaP u) {
 }
 
 // ---- the instantiations live in three translation units (umma_q4.cu, umma_q8.cu, umma_f16.cu); these tables find them.
-// variant: 0 = (KW 1, lock step), 1 = (KW 2, lock step), 2 = (KW 2, separate token ring); fp16 weights have variant 0 only.
+// variant: 0 = (KW 1, lock step), 1 = (KW 2, lock step), 2 = (KW 2, separate token ring), 3 = (KW 4,
+// separate), 4 = (KW 1, pair of blocks); fp16 weights: KW 1 in lock step, alone or as a pair.
 typedef void (*umma_kernel_fn)(const UmmaP, const CUtensorMap, const CUtensorMap);
 typedef void (*umma_finish_fn)(const UmmaP);
 umma_kernel_fn umma_kernel_q4(uint32_t variant, uint32_t epi);
 umma_kernel_fn umma_kernel_q8(uint32_t variant, uint32_t epi);
-umma_kernel_fn umma_kernel_f16(uint32_t epi);
+umma_kernel_fn umma_kernel_f16(uint32_t pair, uint32_t epi);
 umma_finish_fn umma_finish_kernel(uint32_t epi);
-#define P0P_UMMA_ROW(ENC, KW, LOCK) {k_gemm_umma<ENC, P0P_EPI_F16, KW, LOCK>, k_gemm_umma<ENC, P0P_EPI_F32, KW, LOCK>, k_gemm_umma<ENC, P0P_EPI_RESADD, KW, LOCK>, \
-                                     k_gemm_umma<ENC, P0P_EPI_SWIGLU, KW, LOCK>, k_gemm_umma<ENC, P0P_EPI_HEADS, KW, LOCK>, k_gemm_umma<ENC, P0P_EPI_BIAS, KW, LOCK>, \
-                                     k_gemm_umma<ENC, P0P_EPI_ONORMGATE, KW, LOCK>}
+#define P0P_UMMA_ROW(ENC, KW, LOCK, PAIR) {k_gemm_umma<ENC, P0P_EPI_F16, KW, LOCK, PAIR>, k_gemm_umma<ENC, P0P_EPI_F32, KW, LOCK, PAIR>, k_gemm_umma<ENC, P0P_EPI_RESADD, KW, LOCK, PAIR>, \
+                                     k_gemm_umma<ENC, P0P_EPI_SWIGLU, KW, LOCK, PAIR>, k_gemm_umma<ENC, P0P_EPI_HEADS, KW, LOCK, PAIR>, k_gemm_umma<ENC, P0P_EPI_BIAS, KW, LOCK, PAIR>, \
+                                     k_gemm_umma<ENC, P0P_EPI_ONORMGATE, KW, LOCK, PAIR>}
 
 }  // namespace p0p

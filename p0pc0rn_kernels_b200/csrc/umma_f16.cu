@@ -3,9 +3,9 @@
 
 namespace p0p {
 
-umma_kernel_fn umma_kernel_f16(uint32_t epi) {
-  static const umma_kernel_fn table[7] = P0P_UMMA_ROW(P0P_ENC_F16, 1, true);
-  return table[epi];
+umma_kernel_fn umma_kernel_f16(uint32_t pair, uint32_t epi) {
+  static const umma_kernel_fn table[2][7] = {P0P_UMMA_ROW(P0P_ENC_F16, 1, true, false), P0P_UMMA_ROW(P0P_ENC_F16, 1, true, true)};
+  return table[pair][epi];
 }
 
 umma_finish_fn umma_finish_kernel(uint32_t epi) {

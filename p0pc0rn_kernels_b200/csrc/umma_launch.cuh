@@ -154,8 +154,9 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   // total by the cost model below wins.
   const bool atm = p.enc != P0P_ENC_F16;
   const uint32_t ncols = (p.epi == P0P_EPI_SWIGLU || p.epi == P0P_EPI_HEADS || p.epi == P0P_EPI_ONORMGATE) ? p.N : ((p.N + 3u) & ~3u);
-  u.n_tiles = (ncols + 127u) / 128u;
+  u.nt_all = (ncols + 127u) / 128u;
   const uint32_t bt_max = atm ? 384u : 256u, KSn = p.K / 64u;
+  const uint64_t epi_tok = (p.epi == P0P_EPI_HEADS || p.epi == P0P_EPI_ONORMGATE) ? 150u : p.epi == P0P_EPI_SWIGLU ? 30u : 24u;      // cycles of epilogue per token of a tile
   uint32_t BT;
   if (is_conv) { u.cvR = conv_tile_rows(p, atm); BT = u.cvR * p.Wo; }
   else if (p.M <= 256u) BT = std::max(16u, (p.M + 15u) & ~15u);
@@ -163,11 +164,10 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
     double best = 1e300; BT = 0;
     for (uint32_t cand = bt_max; cand >= 128u; cand -= 16u) {
       if (cand > 256u && cand % 32u) continue;
-      const uint64_t t = (uint64_t)u.n_tiles * ((p.M + cand - 1u) / cand);
+      const uint64_t t = (uint64_t)u.nt_all * ((p.M + cand - 1u) / cand);
       // measured: a k-step costs ~750 cycles up to 256 tokens (four dependent multiplies, or the dequantisation) and
       // ~2.5 cycles per token beyond; a single-accumulator tile exposes its epilogue, whose cost per token depends on the kind
       const uint64_t kstep = std::max<uint64_t>(5u * cand / 2u, atm ? 750u : 720u);
-      const uint64_t epi_tok = (p.epi == P0P_EPI_HEADS || p.epi == P0P_EPI_ONORMGATE) ? 150u : p.epi == P0P_EPI_SWIGLU ? 30u : 24u;
       // (with two accumulators the epilogue hides behind the next tile's k loop unless it is the longer of the two; it runs
       // about half as fast there, sharing the issue slots with the dequantisation)
       const uint64_t per_tile = (atm && cand > 128u) ? (uint64_t)KSn * kstep + epi_tok * cand : std::max<uint64_t>((uint64_t)KSn * kstep, 2u * epi_tok * cand);
@@ -178,43 +178,80 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
       if (rounds * (double)per_tile < best) { best = rounds * (double)per_tile; BT = cand; }
     }
   }
-  // ---- tensor memory (512 columns).  fp16 weights: two accumulator buffers of 256 columns.  Quantised weights: the accumulators
-  // first, the dequantised operand's stages in all the columns behind them.  Two accumulator buffers (the next tile's multiplies
-  // overlap the epilogue) for tiles up to 128 tokens, one beyond.  Every hand-over between the roles is a round trip of several
-  // hundred cycles, so the number of operand stages in flight, not the conversion or the multiplies, is what bounds narrow and
-  // medium tiles: they get every column the accumulators leave.  (Consecutive multiplies into one accumulator issue back to back
-  // at the tensor pipe's rate, so a tile has ONE accumulator: KSPLIT stays 1.)
-  u.BT = BT; u.KSPLIT = 1u;
-  u.NACC = atm ? (BT <= 128u ? 2u : 1u) : (BT > 256u ? 1u : 2u);
-  u.m_tiles = (p.M + BT - 1u) / BT;
   // ---- split-K: when the tiles leave SMs idle (few output columns) or the last round is nearly empty, each tile's k loop
   // is cut into S units whose fp32 partial sums a second kernel adds.  Never for conv3 (S would depend on M, and chunked
-  // and whole-clip calls must add in the same order).
-  const uint32_t tiles_all = u.n_tiles * u.m_tiles;
-  u.S = 1u; u.ks_per = KSn; u.T0 = tiles_all;
-  if (p.xmode != P0P_X_CONV3) {
-    const uint64_t tiles = tiles_all;
-    const uint64_t kstep = std::max<uint64_t>(5u * BT / 2u, 750u), epi = 24u * BT;
-    const uint64_t whole = KSn * kstep + (u.NACC == 1u ? epi : 0u);                  // one unsplit tile
-    uint64_t best = ((tiles + sms - 1) / sms) * whole;
+  // and whole-clip calls must add in the same order).  nb: blocks per tile; kstep: cycles per 64 k; exposed: of a tile's epilogue.
+  struct Split { uint32_t S, per, T0; uint64_t cost; };
+  auto split = [&](uint32_t nb, uint32_t bt, uint64_t kstep, uint64_t exposed) {
+    const uint64_t tiles = (uint64_t)((u.nt_all + nb - 1u) / nb) * ((p.M + bt - 1u) / bt), slots = sms / nb, epi = 24u * bt;
+    const uint64_t whole = KSn * kstep + exposed;                                    // one unsplit tile
+    Split r{1u, KSn, (uint32_t)tiles, ((tiles + slots - 1) / slots) * whole};
+    if (p.xmode == P0P_X_CONV3) return r;
     // (a) every tile split (few tiles)
     for (uint32_t S = 2u; S <= 16u; S++) {
       const uint32_t per = (KSn + S - 1u) / S;
       if (per < 8u || (uint64_t)(S - 1u) * per >= KSn) continue;                     // every unit gets k-steps, at least 8 each
-      const uint64_t cost = ((tiles * S + sms - 1) / sms) * (per * kstep + epi + 3000u) + 6000u + (uint64_t)S * BT * 40u;   // + pipeline fill per unit; second kernel: launch, partials written and read
-      if (cost * 20u < best * 19u) { best = cost; u.S = S; u.ks_per = per; u.T0 = 0u; }
+      const uint64_t cost = ((tiles * S + slots - 1) / slots) * (per * kstep + epi + 3000u) + 6000u + S * bt * std::max<uint64_t>(40u, tiles * nb / 12u) + epi_tok * bt * tiles * nb / (2u * sms);   // + pipeline fill per unit; second kernel: launch, partials read, epilogue
+      if (cost * 20u < r.cost * 19u) r = Split{S, per, 0u, cost};
     }
     // (b) only the tiles of the last round split over the SMs that round would leave idle
-    const uint64_t t0 = (tiles / sms) * sms, tail = tiles - t0;
+    const uint64_t t0 = (tiles / slots) * slots, tail = tiles - t0;
     if (t0 && tail) {
       for (uint32_t S = 2u; S <= 16u; S++) {
         const uint32_t per = (KSn + S - 1u) / S;
         if (per < 4u || (uint64_t)(S - 1u) * per >= KSn) continue;
-        const uint64_t cost = (t0 / sms) * whole + ((tail * S + sms - 1) / sms) * (per * kstep + epi + 3000u) + 6000u;
-        if (cost * 20u < best * 19u) { best = cost; u.S = S; u.ks_per = per; u.T0 = (uint32_t)t0; }
+        const uint64_t cost = (t0 / slots) * whole + ((tail * S + slots - 1) / slots) * (per * kstep + epi + 3000u) + 6000u;
+        if (cost * 20u < r.cost * 19u) r = Split{S, per, (uint32_t)t0, cost};
+      }
+    }
+    return r;
+  };
+  u.NACC = atm ? (BT <= 128u ? 2u : 1u) : (BT > 256u ? 1u : 2u);
+  Split sp = split(1u, BT, std::max<uint64_t>(5u * BT / 2u, 750u), u.NACC == 1u ? 24u * BT : 0u);
+  // ---- a pair of blocks per tile of 256 columns, or blocks on their own?  Up to 160 tokens a lone block's shared memory keeps up
+  // (q8, 130 x 14336 x 4096: 24.3 us alone, 25.0 as a pair).  Above, both plans are priced with what a 64-k step costs on a busy
+  // GPU (cycles, from the rounds and steps of whole calls at K = 4096): alone 3.25 per token (975 at least), fp16 weights
+  // 358 + 2.8 per token; a pair 190 + 2.75 per token (620 at least, the conversion), fp16 weights 190 + 3.1, and 3.1 to 3.3 where
+  // the tile takes two multiplies (above 256 tokens, steps of 64).  A pair's tiles up to 192 tokens have two accumulators, so the
+  // next tile's multiplies hide the epilogue: what the head epilogue wants (150 cycles a token; q8, 3600 x 9216 x 3072 with it: 242 us
+  // alone, 235 with 320 tokens, 214 with 192).  gate/up of the LLM block at 512 tokens: 111.5 alone, 101.2 as a pair of 256 tokens;
+  // fp16 16384 x 512 x 4608: 88 and 74.5.  A convolution's tile is given (bits must not depend on it): a pair wherever its rows split.
+  bool pair = false;
+  if (u.nt_all >= 2u && sms % 2u == 0u && p.M > 160u) {
+    if (is_conv) {
+      const uint32_t m = BT > 256u ? 4u : 2u;                                          // (whole image rows to each block's share of each multiply, 32 tokens to a multiply)
+      if (u.cvR % m == 0u && BT % (16u * m) == 0u) { pair = true; sp = split(2u, BT, atm ? std::max(620u, 190u + 11u * BT / 4u) : 190u + 31u * BT / 10u, BT > 192u && atm ? epi_tok * BT : 0u); }
+    } else {
+      const uint64_t alone = BT <= 128u ? 750u : atm ? std::max<uint64_t>(13u * BT / 4u, 975u) : 358u + 14u * BT / 5u;
+      uint64_t best = split(1u, BT, alone, u.NACC == 1u ? epi_tok * BT : 0u).cost;
+      const uint32_t top = std::min(bt_max, p.M <= 256u ? (p.M + 31u) & ~31u : bt_max);
+      for (uint32_t cand = top; cand >= std::min(top, 160u); cand -= 32u) {
+        if (cand > 256u && cand % 64u) continue;
+        const uint64_t kstep = cand > 256u ? (cand > 320u ? 31u : 33u) * cand / 10u : atm ? std::max(620u, 190u + 11u * cand / 4u) : 190u + 31u * cand / 10u;
+        const bool two = !atm || cand <= 192u;
+        const uint64_t hidden = 17u * epi_tok * cand / 10u, exposed = !two ? epi_tok * cand : hidden > KSn * kstep ? hidden - KSn * kstep : 0u;
+        const Split q = split(2u, cand, kstep, exposed);
+        if (q.cost < best) { best = q.cost; sp = q; BT = cand; pair = true; }
       }
     }
   }
+#ifdef P0P_KNOBS
+  if (const char* e = getenv("P0P_PAIR")) if (!atoi(e)) pair = false;
+#endif
+  u.PAIR = pair ? 1u : 0u;
+  u.n_tiles = pair ? (u.nt_all + 1u) / 2u : u.nt_all;
+  const uint32_t NB = 1u + u.PAIR, slots = sms / NB;                                 // blocks of a tile, tiles that run side by side
+  // ---- tensor memory (512 columns).  fp16 weights: two accumulator buffers of 256 columns.  Quantised weights: the accumulators
+  // first, the dequantised operand's stages in all the columns behind them.  Two accumulator buffers (the next tile's multiplies
+  // overlap the epilogue) for tiles up to 128 tokens (pairs: 192), one beyond.  Every hand-over between the roles is a round trip of
+  // several hundred cycles, so the number of operand stages in flight, not the conversion or the multiplies, is what bounds narrow
+  // and medium tiles: they get every column the accumulators leave.  (Consecutive multiplies into one accumulator issue back to back
+  // at the tensor pipe's rate, so a tile has ONE accumulator.)
+  u.BT = BT;
+  u.NACC = atm ? (BT <= (pair ? 192u : 128u) ? 2u : 1u) : (BT > 256u ? 1u : 2u);
+  u.m_tiles = (p.M + BT - 1u) / BT;
+  const uint32_t tiles_all = u.n_tiles * u.m_tiles;
+  u.S = sp.S; u.ks_per = sp.per; u.T0 = sp.T0;
   // pipeline step: 128 k for quantised weights up to 256 tokens (the hand-over costs dominate there), 64 k otherwise (wide tiles
   // are bound by the multiplies and their stages are large; fp16 weights are bound by shared memory).  Depends on the tile only.
   u.KW = (atm && BT <= 256u) ? 2u : 1u;
@@ -228,6 +265,7 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   // weight): two or three such steps would be all fill and drain.
   // (8-bit weights up to 96 tokens: beyond, their 34-KB record stages and the 64-KB token stages leave two of each)
   if (atm && BT <= (p.enc == P0P_ENC_Q4 ? 128u : 96u) && u.ks_per >= 32u) { u.KW = 4u; if (BT > 64u) u.NACC = 1u; }
+  if (pair) { u.KW = 1u; u.NACC = atm ? (BT <= 192u ? 2u : 1u) : 2u; }      // (q4, gate/up at 512 tokens: 128-k steps 103.7 us, 64-k steps 101.2)
 #ifdef P0P_KNOBS      // (tuning experiments only: a library built with -DP0P_KNOBS lets environment variables override the plan)
   if (const char* e = getenv("P0P_NACC")) u.NACC = (uint32_t)atoi(e);
   if (const char* e = getenv("P0P_KW")) u.KW = (uint32_t)atoi(e);
@@ -236,18 +274,18 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   u.a_col0 = atm ? ((u.NACC * BT + 31u) & ~31u) : 512u;
   // Token-ring stages: what shared memory allows for wide tiles; more for narrow ones, whose loads would otherwise be exposed.
   // fp16 weights have no operand ring of their own: the weight tile travels with the tokens (lock step, shared barriers).
-  if (!atm) { u.NS = BT > 192u ? 3u : 4u; u.NA = u.NS; u.LOCK = 1u; }
+  if (!atm) { u.NS = pair ? std::min<uint32_t>(6u, 190u * 1024u / (U_A_BYTES + BT * 64u)) : BT > 192u ? 3u : 4u; u.NA = u.NS; u.LOCK = 1u; }
   else {
     u.NA = std::min<uint32_t>(U_NA_MAX, (512u - u.a_col0) / (32u * u.KW));
     // (shared memory: up to 144 KB of token stages, less where three record stages would not fit beside them)
-    const uint32_t xstage = u.KW * BT * 128u;
+    const uint32_t xstage = u.KW * BT * 128u / NB;
     const uint32_t qst = p.enc == P0P_ENC_Q4 ? UQ<P0P_ENC_Q4>::STAGE : (u.KW == 4u ? UQ<P0P_ENC_Q8, 4>::STAGE : UQ<P0P_ENC_Q8>::STAGE);
     const uint32_t xroom = std::min<uint32_t>(144u * 1024u, 227u * 1024u - 20u * 1024u - 3u * qst);
     u.NS = std::max(2u, std::min<uint32_t>(U_NX_MAX, xroom / xstage));
     u.LOCK = 0u;
     // Tiles above 128 tokens are bound by the multiplies, and there every instruction the issuing warp runs between two
     // multiplies shows: the two rings advance in lock step on shared barriers (one wait, one commit per step).
-    if (u.KW == 1u || BT > 128u) { u.NS = std::min(u.NS, u.NA); u.NA = u.NS; u.LOCK = 1u; }
+    if (u.KW == 1u || BT > 128u || pair) { u.NS = std::min(u.NS, u.NA); u.NA = u.NS; u.LOCK = 1u; }
   }
 #ifdef P0P_KNOBS
   if (const char* e = getenv("P0P_NS")) u.NS = (uint32_t)atoi(e);
@@ -255,16 +293,17 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   if (const char* e = getenv("P0P_LOCK")) u.LOCK = (uint32_t)atoi(e);
   if (u.LOCK) u.NA = u.NS = std::min(u.NS, u.NA);
 #endif
+  if (u.NA < 2u || u.NS < 2u) return fail(c, -12, "gemm: no room for two operand stages of this tile shape");      // (the two dequantisation groups work in two stages)
   // record stages: as many as fit beside the operand stages, up to about 100 KB in flight
   const size_t qstage = p.enc == P0P_ENC_Q4 ? UQ<P0P_ENC_Q4>::STAGE : p.enc == P0P_ENC_Q8 ? (u.KW == 4u ? UQ<P0P_ENC_Q8, 4>::STAGE : UQ<P0P_ENC_Q8>::STAGE) : 0;
-  const size_t fixed = 1024 + (atm ? 0 : (size_t)u.NS * U_A_BYTES) + (size_t)u.NS * u.KW * BT * 128u + (size_t)U_EPI_BYTES + 1024u;
+  const size_t fixed = 1024 + (atm ? 0 : (size_t)u.NS * U_A_BYTES) + (size_t)u.NS * u.KW * BT * 128u / NB + (size_t)U_EPI_BYTES + 1024u;
   size_t q_cap = 100 * 1024;
 #ifdef P0P_KNOBS
   if (const char* e = getenv("P0P_QCAP")) q_cap = (size_t)atoi(e) * 1024;
 #endif
   u.NQ = qstage ? (uint32_t)std::min<size_t>(std::min<size_t>(U_NQ_MAX, (q_cap + qstage - 1) / qstage), (227 * 1024 - fixed) / qstage) : 0u;
   if (qstage && u.NQ < 2u) return fail(c, -12, "gemm: no room for the record stages of this tile shape");
-  const uint64_t sk_bytes = u.S > 1u ? (uint64_t)u.S * (tiles_all - u.T0) * BT * 128u * 4u : 0u;
+  const uint64_t sk_bytes = u.S > 1u ? (uint64_t)u.S * (tiles_all - u.T0) * NB * BT * 128u * 4u : 0u;
   if (pro_bytes + sk_bytes) {
     if (int r = ensure_scratch(c, pro_bytes + sk_bytes + 256)) return r;
   }
@@ -288,42 +327,46 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   }
   u.sk_part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(c->scratch) + pro_bytes);
   {   // a wave of `sms` tiles reads G token tiles and sms / G weight tiles: least bytes at G = sqrt(sms * weight tile / token tile)
-    const double wt = 128.0 * (p.enc == P0P_ENC_Q4 ? 0.625 : p.enc == P0P_ENC_Q8 ? 1.03125 : 2.0), xt = 2.0 * BT;
-    const double g = std::sqrt((double)sms * wt / xt);
+    const double wt = 128.0 * NB * (p.enc == P0P_ENC_Q4 ? 0.625 : p.enc == P0P_ENC_Q8 ? 1.03125 : 2.0), xt = 2.0 * BT;
+    const double g = std::sqrt((double)slots * wt / xt);
     u.G = (uint32_t)std::min<double>(std::max(1.0, std::floor(g + 0.5)), (double)u.m_tiles);
   }
   u.p = p; u.status = c->dev_status;
   CUtensorMap mx, mw;
   if (p.xmode == P0P_X_CONV3) {
     const uint32_t frames = p.ks > 1u ? p.ks : p.stride - p.padL;
-    if (!make_map_clip(&mx, xbase, p.Ci, p.Wi, p.Hi, frames, p.Wo, BT > 256u ? u.cvR / 2u : u.cvR)) return fail(c, -12, "gemm: the clip tensor map could not be encoded");
+    if (!make_map_clip(&mx, xbase, p.Ci, p.Wi, p.Hi, frames, p.Wo, (BT > 256u ? u.cvR / 2u : u.cvR) / NB)) return fail(c, -12, "gemm: the clip tensor map could not be encoded");
   } else if (p.xmode == P0P_X_CONV) {
-    if (!make_map_clip(&mx, xbase, p.Ci, p.Wi, p.Hi, 1u, p.Wo, BT > 256u ? u.cvR / 2u : u.cvR, p.stride)) return fail(c, -12, "gemm: the image tensor map could not be encoded");
-  } else if (!make_map(&mx, xbase, p.K, p.M, xld, BT > 256u ? BT / 2u : BT)) return fail(c, -12, "gemm: the token tensor map could not be encoded");
+    if (!make_map_clip(&mx, xbase, p.Ci, p.Wi, p.Hi, 1u, p.Wo, (BT > 256u ? u.cvR / 2u : u.cvR) / NB, p.stride)) return fail(c, -12, "gemm: the image tensor map could not be encoded");
+  } else if (!make_map(&mx, xbase, p.K, p.M, xld, (BT > 256u ? BT / 2u : BT) / NB)) return fail(c, -12, "gemm: the token tensor map could not be encoded");
   if (p.enc == P0P_ENC_F16) {
     if (!make_map(&mw, reinterpret_cast<const __half*>(p.W) + p.wk0, p.K, p.Nw, p.wG, 128u)) return fail(c, -12, "gemm: the weight tensor map could not be encoded");
   } else mw = mx;
   const size_t qbytes = u.NQ * qstage;
   // at least 120 KB: one block per SM, so that a block never waits for another's tensor memory
-  const size_t smem = std::max<size_t>(120 * 1024, 1024 + (atm ? 0 : (size_t)u.NS * U_A_BYTES) + (size_t)u.NS * u.KW * BT * 128u + qbytes + (size_t)U_EPI_BYTES + 1024u);
-  const int grid = (int)std::min<uint64_t>((uint64_t)u.T0 + (uint64_t)(tiles_all - u.T0) * u.S, sms);
+  const size_t smem = std::max<size_t>(120 * 1024, 1024 + (atm ? 0 : (size_t)u.NS * U_A_BYTES) + (size_t)u.NS * u.KW * BT * 128u / NB + qbytes + (size_t)U_EPI_BYTES + 1024u);
+  const int grid = (int)(NB * std::min<uint64_t>((uint64_t)u.T0 + (uint64_t)(tiles_all - u.T0) * u.S, slots));
   const int smem_max = 227 * 1024;          // the most dynamic shared memory a block may opt into on sm_100
   if (smem > (size_t)smem_max) return fail(c, -12, "gemm: tile configuration needs %zu bytes of shared memory", smem);
-  const uint32_t variant = u.KW == 1u ? 0u : u.KW == 4u ? 3u : u.LOCK ? 1u : 2u;
-  const umma_kernel_fn kern = p.enc == P0P_ENC_Q4 ? umma_kernel_q4(variant, p.epi) : p.enc == P0P_ENC_Q8 ? umma_kernel_q8(variant, p.epi) : umma_kernel_f16(p.epi);
+  const uint32_t variant = !atm ? u.PAIR : pair ? 4u : u.KW == 1u ? 0u : u.KW == 4u ? 3u : u.LOCK ? 1u : 2u;
+  const umma_kernel_fn kern = p.enc == P0P_ENC_Q4 ? umma_kernel_q4(variant, p.epi) : p.enc == P0P_ENC_Q8 ? umma_kernel_q8(variant, p.epi) : umma_kernel_f16(variant, p.epi);
   // the shared-memory ceiling is an attribute of (kernel, device): raised once for each pair
-  static DeviceOnce once[3][4][7];
+  static DeviceOnce once[3][5][7];
   cudaError_t e = cudaSuccess;
   if (once[p.enc][variant][p.epi].run(c->device, [&] { e = cudaFuncSetAttribute(reinterpret_cast<const void*>(kern), cudaFuncAttributeMaxDynamicSharedMemorySize, smem_max); return (int)e; }))
     return cuda_fail(c, e != cudaSuccess ? e : cudaErrorInvalidDevice, "tensor-core kernel attribute");
   const uint32_t plan[8] = {u.BT, u.KW, u.LOCK, u.NS, u.NA, u.NACC, u.S, u.T0};
   std::copy(plan, plan + 8, c->last_plan);
   void* args[3] = {&u, &mx, &mw};
-  if ((e = cudaLaunchKernel(reinterpret_cast<const void*>(kern), dim3(grid), dim3(U_THREADS), args, smem, c->stream)) != cudaSuccess) return cuda_fail(c, e, "tensor-core kernel launch");
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = NB; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(U_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = c->stream; cfg.attrs = at; cfg.numAttrs = pair ? 1u : 0u;
+  if ((e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), args)) != cudaSuccess) return cuda_fail(c, e, "tensor-core kernel launch");
   c->launches += 1;
   if (u.S > 1u) {
     void* fargs[1] = {&u};
-    if ((e = cudaLaunchKernel(reinterpret_cast<const void*>(umma_finish_kernel(p.epi)), dim3(tiles_all - u.T0, (BT + U_EPI_TB - 1u) / U_EPI_TB), dim3(128), fargs, 0, c->stream)) != cudaSuccess)
+    if ((e = cudaLaunchKernel(reinterpret_cast<const void*>(umma_finish_kernel(p.epi)), dim3((tiles_all - u.T0) * NB, (BT + U_EPI_TB - 1u) / U_EPI_TB), dim3(128), fargs, 0, c->stream)) != cudaSuccess)
       return cuda_fail(c, e, "split-K second stage launch");
     c->launches += 1;
   }

@@ -406,6 +406,31 @@ def test_tensor_core_kernel(gpu, oracle, case):
         assert gpu.lastPlan["KW"] == 4 and gpu.lastPlan["S"] == 1, gpu.lastPlan
 
 
+# two blocks per tile: token counts around the steps of 32 and the one / two accumulator and one / two multiply edges, an odd count of
+# 128-column tiles (the last pair's second block has nothing to store) under each kind of epilogue, units of a split k loop
+PAIRS = [
+    dict(name="pair q4 M161", enc="q4", M=161, N=256, K=512),
+    dict(name="pair q8 M192 odd tiles", enc="q8", M=192, N=384, K=256),
+    dict(name="pair q4 M257 odd tiles f32", enc="q4", M=257, N=128 * 5, K=576, epi="f32"),
+    dict(name="pair q8 M224 ragged columns resadd", enc="q8", M=224, N=328, K=320, epi="resadd", w_rows=384),
+    dict(name="pair q4 M512 odd tiles rms+swiglu", enc="q4", M=512, N=2 * 64 * 7, K=1024, xmode="rms", epi="swiglu"),
+    dict(name="pair q8 M400 odd heads lnmod", enc="q8", M=400, N=128 * 9, K=512, xmode="lnmod", epi="heads", heads=dict(Ltot=410, Hq=5, Hkv=2, rowOff=10, eps=1e-6)),
+    dict(name="pair q4 M256 split k, odd tiles", enc="q4", M=256, N=128 * 3, K=4096, epi="resadd"),
+    dict(name="pair f16 M170 bias", enc="f16", M=170, N=256, K=64, epi="bias"),
+    dict(name="pair f16 M513 odd tiles, ring wrap", enc="f16", M=513, N=128 * 3, K=1600),
+    dict(name="pair q4 many tiles", enc="q4", M=1000, N=128 * 150, K=256),
+]
+
+
+@pytest.mark.parametrize("case", PAIRS, ids=lambda c: c["name"])
+def test_pair_tiles(gpu, oracle, case):
+    from p0pc0rn_kernels_b200._lib import K_UMMA
+    h = CS.build(dict(case))
+    got = CS.run_gpu(gpu, h)
+    assert gpu.lastKernel == K_UMMA
+    CS.check(got, CS.run_oracle(h), case["name"])
+
+
 def test_tensor_core_matches_general_kernel_bits_of_weights(gpu, oracle):
     """identity tokens turn the multiply into a read-out of the operand tiles: the tensor-core kernel's dequantised
     weights equal f16(deq) bit for bit (fp32 accumulation of one non-zero product per output is exact)"""
@@ -455,6 +480,27 @@ DECODE = [
     dict(name="d q4 M2 whole-unit ranges (1800 units)", enc="q4", M=2, N=64 * 1800, K=512),
     dict(name="d K not a stage multiple -> general kernel", enc="q4", M=2, N=128, K=384, expect="generic"),
 ]
+
+
+@pytest.mark.parametrize("M", [1, 2, 3, 4])
+@pytest.mark.parametrize("K", [256, 512 + 256, 2048 + 256])
+def test_decode_few_tokens_share_the_columns(gpu, oracle, M, K):
+    """4-bit weights, up to 4 tokens: several scale groups ride in one multiply.  Groups of very different scales (a factor of 2^8 from
+    one group to the next) show a sum that ended in another group's column."""
+    O = oracle
+    N = 192
+    W0 = O.randn(N * K, 5, 0.05).reshape(N, K // 32, 32) * (2.0 ** (-4.0 * (np.arange(K // 32) % 3)))[None, :, None]
+    Wb, deq = CS.encode("q4g32a.t64", W0.reshape(-1).astype(np.float32), N, K)
+    X = O.randn(M * K, 6)
+    ref = P().fromF16(P().toF16(X)).reshape(M, K).astype(np.float64) @ O.from_f16(O.to_f16(deq)).reshape(N, K).astype(np.float64).T
+    wb, xb, yb = gpu.upload(Wb), gpu.upload(P().toF16(X)), gpu.buffer(M * N * 4)
+    try:
+        P().gemm(gpu, {"w": {"enc": "q4g32a.t64", "buf": wb, "off": 0, "bytes": wb._pf, "rows": N, "cols": K}, "x": {"buf": xb}, "y": {"buf": yb}, "M": M, "N": N, "K": K, "epi": "f32", "kernel": "decode"})
+        got = gpu.read(yb, 0, M * N * 4).view(np.float32).reshape(M, N)
+        # the oracle's weights are rounded to fp16, the kernel's are not: 2^-11 relative per weight, uncorrelated
+        assert np.linalg.norm(got - ref) <= 1e-3 * np.linalg.norm(ref)
+    finally:
+        for b in (wb, xb, yb): gpu.free(b)
 
 
 @pytest.mark.parametrize("case", DECODE, ids=lambda c: c["name"])
