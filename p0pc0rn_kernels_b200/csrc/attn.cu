@@ -57,8 +57,7 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
 #ifdef P0P_KNOBS
     if (const char* e = getenv("P0P_ATTN_NS")) { const uint32_t T = (Lq + 127u) / 128u; uint32_t s = (uint32_t)atoi(e); if (s <= T && ((T - s) & 1u) == 0u) { t.ns = s; t.np = (T - s) / 2u; } }
 #endif
-    k_attn_tc<<<Hq * (t.np + t.ns), ATC_THREADS, ATC_SMEM, c->stream>>>(t, mq, mk, mv);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(k_attn_tc, dim3(Hq * (t.np + t.ns)), dim3(ATC_THREADS), ATC_SMEM, c->stream, t, mq, mk, mv);
     if (e != cudaSuccess) return cuda_fail(c, e, "attention launch");
     c->launches += 1;
     c->last_kernel = P0P_K_ATTN_TMEM;
@@ -81,8 +80,7 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
   int rc = once[wm == 4u ? 3 : wm].run(c->device, [&] { return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM); });
   if (rc) return cuda_fail(c, (cudaError_t)rc, "attention kernel attribute");
   if (Hkv > 65535u || rbs > 65535u) return fail(c, -5, "attention: at most 65535 kv heads and 65535 blocks of query rows");
-  kern<<<dim3(S, Hkv, rbs), 128, AT_SMEM, c->stream>>>(p);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(kern, dim3(S, Hkv, rbs), dim3(128), AT_SMEM, c->stream, p);
   if (e != cudaSuccess) return cuda_fail(c, e, "attention launch");
   c->launches += 1;
   c->last_kernel = P0P_K_ATTN_WARP;

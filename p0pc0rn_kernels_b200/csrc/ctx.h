@@ -80,4 +80,18 @@ struct DeviceGuard {
 
 int ensure_scratch(p0p_ctx* c, uint64_t bytes);
 
+// Launch as a programmatic dependent of whatever precedes in the stream: the kernel may start while that one drains, and sets itself
+// up meanwhile.  A kernel launched so calls grid_dependency_wait() before it touches what an earlier kernel may write, and
+// grid_launch_dependents() only after that wait (so that the kernel after it never overlaps the one before it).  Worth one to two
+// microseconds at each boundary between kernels: LLM block at 16 tokens (5 kernels) 75 -> 64 us, at 512 tokens 200 -> 190, 32:8 heads 1000
+// causal tokens 23.6 -> 20.6, one query over 4000 keys 10.4 -> 8.9, GroupNorm + convolution (4 kernels) 102 -> 97.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = st; cfg.attrs = at; cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k, P(args)...);
+}
+
 }  // namespace p0p

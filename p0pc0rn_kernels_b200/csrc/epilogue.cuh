@@ -4,6 +4,7 @@
 // Arithmetic as in the reference shader, src/ops/gemm.js:191-254.
 #pragma once
 #include "common.cuh"
+#include "sync.cuh"
 
 namespace p0p {
 
@@ -105,7 +106,7 @@ __device__ __forceinline__ void epilogue_cols(const KP& p, uint32_t m0, uint32_t
       const uint32_t ang = half_mode ? (c & 63u) : (c >> 1);
 #pragma unroll
       for (int j = 0; j < TB; j++) {
-        const float2 t = __ldg(reinterpret_cast<const float2*>(p.RP + ((size_t)p.rowOff + min(m0 + j, p.M - 1u)) * 128u) + ang);
+        const float2 t = ld_now(reinterpret_cast<const float2*>(p.RP + ((size_t)p.rowOff + min(m0 + j, p.M - 1u)) * 128u) + ang);
         cs[j] = t.x; sn[j] = t.y;
       }
     }
@@ -139,7 +140,7 @@ __device__ __forceinline__ void epilogue_cols(const KP& p, uint32_t m0, uint32_t
         }
       }
       bar_sync_named(barid, 128);
-      const float nw = __ldg(p.EV + p.evOff + (sec == 1u ? 128u : 0u) + c);
+      const float nw = ld_now(p.EV + p.evOff + (sec == 1u ? 128u : 0u) + c);
       if (TB % 4 == 0) {
 #pragma unroll
         for (int j = 0; j < TB; j += 4) {
@@ -207,7 +208,7 @@ __device__ __forceinline__ void epilogue_cols(const KP& p, uint32_t m0, uint32_t
     // finishes tokens j = 0, 2, .., the odd lane j = 1, 3, .., each getting the other half of its pair by one shuffle.
     const uint32_t o = col >> 1;
     float gB = 0.0f, uB = 0.0f;
-    if ((p.flags & P0P_F_BIAS) && col < p.N) { gB = __ldg(p.BV + p.bvOff + o); uB = __ldg(p.BV + p.bvOff + p.bvUp + o); }
+    if ((p.flags & P0P_F_BIAS) && col < p.N) { gB = ld_now(p.BV + p.bvOff + o); uB = ld_now(p.BV + p.bvOff + p.bvUp + o); }
     // the activation is chosen outside the token loop: inside it the compiler evaluates both branches per element
     if (p.flags & P0P_F_GELU) swiglu_tokens<TB, true>(p, m0, col, c, acc, gB, uB, sh, vec, par);
     else swiglu_tokens<TB, false>(p, m0, col, c, acc, gB, uB, sh, vec, par);
@@ -220,7 +221,7 @@ __device__ __forceinline__ void epilogue_cols(const KP& p, uint32_t m0, uint32_t
   if (vec) {
     const uint32_t valid = nB < p.N ? min(128u, p.N - nB) : 0u;
     if (epi == P0P_EPI_F16 || epi == P0P_EPI_BIAS) {
-      const float bias = (epi == P0P_EPI_BIAS && col < p.N) ? __ldg(p.EV + p.evOff + col) : 0.0f;
+      const float bias = (epi == P0P_EPI_BIAS && col < p.N) ? ld_now(p.EV + p.evOff + col) : 0.0f;
       __half* st = reinterpret_cast<__half*>(sh) + par * TB * 128;
 #pragma unroll
       for (int j = 0; j < TB; j++) st[j * 128 + c] = __float2half_rn(acc[j] + bias);
@@ -237,8 +238,8 @@ __device__ __forceinline__ void epilogue_cols(const KP& p, uint32_t m0, uint32_t
       if (epi == P0P_EPI_RESADD && live) {
 #pragma unroll
         for (int q = 0; q < 4; q++) {
-          if (p.flags & P0P_F_GATE) g4[q] = __ldg(p.EV + p.evOff + c4 + q);
-          if (p.flags & P0P_F_BIAS) b4[q] = __ldg(p.BV + p.bvOff + c4 + q);
+          if (p.flags & P0P_F_GATE) g4[q] = ld_now(p.EV + p.evOff + c4 + q);
+          if (p.flags & P0P_F_BIAS) b4[q] = ld_now(p.BV + p.bvOff + c4 + q);
         }
       }
       float4 old[TB / 4];
@@ -263,9 +264,9 @@ __device__ __forceinline__ void epilogue_cols(const KP& p, uint32_t m0, uint32_t
   if ((col & ~3u) >= p.N) return;                                   // stores go in groups of four columns (:196)
   float gate = 1.0f, bias = 0.0f;
   if (epi == P0P_EPI_RESADD) {
-    if (p.flags & P0P_F_GATE) gate = __ldg(p.EV + p.evOff + col);
-    if (p.flags & P0P_F_BIAS) bias = __ldg(p.BV + p.bvOff + col);
-  } else if (epi == P0P_EPI_BIAS) bias = __ldg(p.EV + p.evOff + col);
+    if (p.flags & P0P_F_GATE) gate = ld_now(p.EV + p.evOff + col);
+    if (p.flags & P0P_F_BIAS) bias = ld_now(p.BV + p.bvOff + col);
+  } else if (epi == P0P_EPI_BIAS) bias = ld_now(p.EV + p.evOff + col);
   // read-modify-write epilogues fetch all TB old values first (TB loads in flight), then add and store
   float old[TB];
   const bool rmw32 = epi == P0P_EPI_RESADD && !(p.flags & P0P_F_STORE), rmw16 = epi == P0P_EPI_BIAS && (p.flags & P0P_F_RES);

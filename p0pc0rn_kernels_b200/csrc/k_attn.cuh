@@ -16,6 +16,8 @@
 #include <cuda_fp16.h>
 #include <stdint.h>
 
+#include "sync.cuh"
+
 namespace p0p {
 
 struct AttnP {
@@ -79,6 +81,8 @@ __global__ void __launch_bounds__(128) k_attn_split(const AttnP p) {
       at_cp16(dst + AT_TILE_B + o, Vg + src, on);
     }
   };
+  grid_dependency_wait();
+  grid_launch_dependents();
 #pragma unroll
   for (uint32_t s = 0; s < AT_STAGES - 1u; s++) { if (tb + s < te) load(tb + s, s); at_cp_commit(); }
   // this thread's two rows (rows past the end repeat the last one; they are not stored)
@@ -87,7 +91,7 @@ __global__ void __launch_bounds__(128) k_attn_split(const AttnP p) {
 #pragma unroll
   for (int ks = 0; ks < 8; ks++) {
     const uint32_t* a = reinterpret_cast<const uint32_t*>(Qg + (size_t)ra * 128u + ks * 16) + t4; const uint32_t* b = reinterpret_cast<const uint32_t*>(Qg + (size_t)rc * 128u + ks * 16) + t4;
-    qa[ks][0] = __ldg(a); qa[ks][1] = __ldg(b); qa[ks][2] = __ldg(a + 4); qa[ks][3] = __ldg(b + 4);
+    qa[ks][0] = ld_now(a); qa[ks][1] = ld_now(b); qa[ks][2] = ld_now(a + 4); qa[ks][3] = ld_now(b + 4);
   }
   uint32_t lim[2] = {kEnd, kEnd};
   if (p.mode == 1u) { lim[0] = min(p.Lk, min(ra % p.Lq, p.nvalid - 1u) + 1u); lim[1] = min(p.Lk, min(rc % p.Lq, p.nvalid - 1u) + 1u); }

@@ -116,6 +116,8 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
   if (warp == 0) {
     // ================================================================= loads
     if (lane == 0) {
+      grid_dependency_wait();              // (the other roles only touch memory after what is loaded here)
+      grid_launch_dependents();
       mbar_expect_tx(q_full, hasB ? 2u * ATC_TILE : ATC_TILE);
       for (uint32_t t = 0; t < (hasB ? 2u : 1u); t++)
         for (uint32_t c = 0; c < 2u; c++) tma_load_3d(q_sm + t * ATC_TILE + c * 16384u, &mapQ, (int)(c * 64u), (int)(q0 + t * 128u), (int)h, q_full);

@@ -2,6 +2,8 @@
 // row statistics (mean, rstd) the fused norm prologues read (src/ops/misc.js:16-44).
 #pragma once
 #include "common.cuh"
+#include "ctx.h"
+#include "sync.cuh"
 
 namespace p0p {
 
@@ -64,7 +66,7 @@ inline cudaError_t launch_dequant(uint32_t enc, const uint8_t* W, uint32_t wG, u
 // thread's loads are in flight together.  Otherwise (odd alignment, longer rows) the row is read column by column, twice for
 // LayerNorm.  (3600 rows of 3072: 13.8 -> 12.6 us)
 template <bool VEC>
-__global__ void __launch_bounds__(256) k_rowstats(const float* __restrict__ X, uint32_t ld, uint32_t c0, uint32_t cols, uint32_t mode, float eps, float* __restrict__ ST) {
+__global__ void __launch_bounds__(256) k_rowstats(const float* X, uint32_t ld, uint32_t c0, uint32_t cols, uint32_t mode, float eps, float* ST) {
   __shared__ float red[2][8];
   const uint32_t row = blockIdx.x, t = threadIdx.x;
   const float* x = X + (size_t)row * ld + c0;
@@ -79,10 +81,12 @@ __global__ void __launch_bounds__(256) k_rowstats(const float* __restrict__ X, u
     return s;
   };
   float mean = 0.0f, q = 0.0f;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (VEC) {
     float4 v[8];
 #pragma unroll
-    for (uint32_t i = 0; i < 8u; i++) { const uint32_t k = (i * 256u + t) * 4u; v[i] = k < cols ? __ldg(reinterpret_cast<const float4*>(x + k)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+    for (uint32_t i = 0; i < 8u; i++) { const uint32_t k = (i * 256u + t) * 4u; v[i] = k < cols ? ld_now(reinterpret_cast<const float4*>(x + k)) : make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
     if (mode == 0u) {
       float s = 0.0f;
 #pragma unroll
@@ -105,8 +109,7 @@ __global__ void __launch_bounds__(256) k_rowstats(const float* __restrict__ X, u
 
 inline cudaError_t launch_rowstats(const float* X, uint32_t ld, uint32_t c0, uint32_t rows, uint32_t cols, uint32_t mode, float eps, float* ST, cudaStream_t st) {
   const bool vec = cols % 4u == 0u && cols <= 8192u && ((uintptr_t)(X + c0) & 15u) == 0u && (ld % 4u == 0u || rows == 1u);
-  (vec ? k_rowstats<true> : k_rowstats<false>)<<<rows, 256, 0, st>>>(X, ld, c0, cols, mode, eps, ST);
-  return cudaGetLastError();
+  return launch_chained(vec ? k_rowstats<true> : k_rowstats<false>, dim3(rows), dim3(256), 0, st, X, ld, c0, cols, mode, eps, ST);
 }
 
 }  // namespace p0p

@@ -107,7 +107,7 @@ __device__ __forceinline__ void d_stage_tokens(const DecodeP& d, uint32_t kb0, u
     if (XMODE == P0P_X_F16) {
       const __half* src = reinterpret_cast<const __half*>(p.X) + (size_t)m * p.ldx + p.kx0 + k0;
       if (p.vecx) {
-        const uint4 u = __ldg(reinterpret_cast<const uint4*>(src));
+        const uint4 u = ld_now(reinterpret_cast<const uint4*>(src));
         const __half2* h = reinterpret_cast<const __half2*>(&u);
 #pragma unroll
         for (int i = 0; i < 4; i++) { const float2 f = __half22float2(h[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
@@ -119,16 +119,16 @@ __device__ __forceinline__ void d_stage_tokens(const DecodeP& d, uint32_t kb0, u
       // (the host admits this kernel only when x rows and the vector are 16-byte aligned: see decode_supported)
       const float* src = reinterpret_cast<const float*>(p.X) + (size_t)m * p.ldx + p.kx0 + k0;
       const size_t sr = ((size_t)p.statOff + m) * 2u;
-      const float mean = __ldg(p.ST + sr), rstd = __ldg(p.ST + sr + 1);
+      const float mean = ld_now(p.ST + sr), rstd = ld_now(p.ST + sr + 1);
       const float* pv = p.PV + p.pvOff + p.kx0 + k0;
       float xv[8], g1[8], g2[8];
       if (d.vec32) {
-        *reinterpret_cast<float4*>(xv) = __ldg(reinterpret_cast<const float4*>(src)); *reinterpret_cast<float4*>(xv + 4) = __ldg(reinterpret_cast<const float4*>(src) + 1);
-        *reinterpret_cast<float4*>(g1) = __ldg(reinterpret_cast<const float4*>(pv)); *reinterpret_cast<float4*>(g1 + 4) = __ldg(reinterpret_cast<const float4*>(pv) + 1);
-        if (XMODE == P0P_X_LNMOD) { *reinterpret_cast<float4*>(g2) = __ldg(reinterpret_cast<const float4*>(pv + p.pvStride)); *reinterpret_cast<float4*>(g2 + 4) = __ldg(reinterpret_cast<const float4*>(pv + p.pvStride) + 1); }
+        *reinterpret_cast<float4*>(xv) = ld_now(reinterpret_cast<const float4*>(src)); *reinterpret_cast<float4*>(xv + 4) = ld_now(reinterpret_cast<const float4*>(src) + 1);
+        *reinterpret_cast<float4*>(g1) = ld_now(reinterpret_cast<const float4*>(pv)); *reinterpret_cast<float4*>(g1 + 4) = ld_now(reinterpret_cast<const float4*>(pv) + 1);
+        if (XMODE == P0P_X_LNMOD) { *reinterpret_cast<float4*>(g2) = ld_now(reinterpret_cast<const float4*>(pv + p.pvStride)); *reinterpret_cast<float4*>(g2 + 4) = ld_now(reinterpret_cast<const float4*>(pv + p.pvStride) + 1); }
       } else {
 #pragma unroll
-        for (int i = 0; i < 8; i++) { xv[i] = __ldg(src + i); g1[i] = __ldg(pv + i); if (XMODE == P0P_X_LNMOD) g2[i] = __ldg(pv + p.pvStride + i); }
+        for (int i = 0; i < 8; i++) { xv[i] = ld_now(src + i); g1[i] = ld_now(pv + i); if (XMODE == P0P_X_LNMOD) g2[i] = ld_now(pv + p.pvStride + i); }
       }
 #pragma unroll
       for (int i = 0; i < 8; i++) {

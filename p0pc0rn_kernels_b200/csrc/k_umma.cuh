@@ -213,6 +213,10 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
   if (warp == 0) {
     // ================================================================= producer of the token tiles (and fp16 weight tiles)
     if (lane == 0) {
+      // (the records of quantised weights stream from the start; tokens, fp16 weights and everything the epilogue touches wait for the
+      // kernel before this one)
+      grid_dependency_wait();
+      grid_launch_dependents();
       Ring r(NS);
       bool ok = true;
       auto load2 = [&](uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar) { if (PAIR) tma_load_2d_pair(dst, m, x, y, bar); else tma_load_2d(dst, m, x, y, bar); };
@@ -342,6 +346,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     // ================================================================= epilogue (TMEM lanes 32*(warp%4) .. +31)
     const uint32_t q = warp & 3u, c = q * 32u + lane;
     uint32_t tl = 0, pass = 0;
+    grid_dependency_wait();
     bool ok = true;
     const bool vec = epilogue_vec_ok(p);
     auto acc_free = [&](uint32_t b) { if (PAIR) mbar_arrive_cluster(cluster_addr(acc_empty + 8u * b, 0u)); else mbar_arrive(acc_empty + 8u * b); };
@@ -488,6 +493,8 @@ __global__ void __launch_bounds__(128) k_umma_finish(const UmmaP u) {
   uint32_t nt, mt; tile_coords(u, u.T0 + t / NB, nt, mt);
   nt = nt * NB + t % NB;
   const uint32_t r0 = blockIdx.y * U_EPI_TB, m0 = mt * u.BT + r0;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (m0 >= p.M || nt >= u.nt_all) return;
   float acc[U_EPI_TB];
 #pragma unroll

@@ -4,21 +4,24 @@
 // for the exact two-pass variance).
 #include "common.cuh"
 #include "ctx.h"
+#include "sync.cuh"
 
 using namespace p0p;
 
 namespace {
 
 // ---- pixstats: R[ro + v] = rsqrt(sum_c x[v][c]^2 / C + eps), x fp16 [V][C].  L lanes share a voxel (16-byte loads).
-__global__ void __launch_bounds__(256) k_pixstats(const __half* __restrict__ X, uint32_t V, uint32_t C, uint32_t L, float eps, float* __restrict__ R, uint32_t vec) {
+__global__ void __launch_bounds__(256) k_pixstats(const __half* X, uint32_t V, uint32_t C, uint32_t L, float eps, float* R, uint32_t vec) {
   const uint32_t gt = blockIdx.x * blockDim.x + threadIdx.x, sub = gt % L;
   const uint32_t v = gt / L;
   float s = 0.0f;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (v < V) {
     const __half* x = X + (size_t)v * C;
     if (vec) {
       for (uint32_t c = sub * 8u; c < C; c += L * 8u) {
-        const uint4 q = __ldg(reinterpret_cast<const uint4*>(x + c));
+        const uint4 q = ld_now(reinterpret_cast<const uint4*>(x + c));
         const __half2* h = reinterpret_cast<const __half2*>(&q);
 #pragma unroll
         for (int i = 0; i < 4; i++) { const float2 f = __half22float2(h[i]); s = fmaf(f.x, f.x, s); s = fmaf(f.y, f.y, s); }
@@ -38,7 +41,7 @@ __global__ void __launch_bounds__(256) k_pixstats(const __half* __restrict__ X, 
 // fixed order (deterministic).  NI = C / 32 rounds make the chunk (NI is a template argument): all of a thread's 16-byte loads are
 // issued before the first is used and the values stay in registers for the second pass.  (128 x 128 x 512: 10.5 -> 8.3 us)
 template <int NI>
-__global__ void __launch_bounds__(256) k_gn_partial(const __half* __restrict__ X, uint32_t pix, uint32_t wgOff, float4* __restrict__ PT) {
+__global__ void __launch_bounds__(256) k_gn_partial(const __half* X, uint32_t pix, uint32_t wgOff, float4* PT) {
   constexpr uint32_t C = 32u * NI, cpg = NI, reps = 2048u / C, per = C / 8u;
   __shared__ float part[256][9];      // per thread, per element of its 8 (padded against bank conflicts)
   __shared__ float chs[C];            // per channel
@@ -47,9 +50,11 @@ __global__ void __launch_bounds__(256) k_gn_partial(const __half* __restrict__ X
   const uint32_t n = npx * C, c0 = (t * 8u) % C;
   const __half* x = X + (size_t)px0 * C;
   const float cnt = (float)(npx * cpg);
+  grid_dependency_wait();
+  grid_launch_dependents();
   uint4 v[NI];
 #pragma unroll
-  for (uint32_t i = 0; i < (uint32_t)NI; i++) { const uint32_t e = i * 2048u + t * 8u; v[i] = e < n ? __ldg(reinterpret_cast<const uint4*>(x + e)) : make_uint4(0u, 0u, 0u, 0u); }
+  for (uint32_t i = 0; i < (uint32_t)NI; i++) { const uint32_t e = i * 2048u + t * 8u; v[i] = e < n ? ld_now(reinterpret_cast<const uint4*>(x + e)) : make_uint4(0u, 0u, 0u, 0u); }
   float acc[8];
   auto reduce_groups = [&](float* out32) {      // acc[] of all threads -> out32[g]; ends with a barrier
 #pragma unroll
@@ -107,13 +112,15 @@ __device__ __forceinline__ Chan chan_merge(Chan a, Chan b) {
   Chan r; r.n = nn; r.mean = a.mean + d * (b.n / nn); r.m2 = a.m2 + b.m2 + d * d * (a.n * b.n / nn);
   return r;
 }
-__global__ void __launch_bounds__(256) k_gn_finalize(const float4* __restrict__ PT, uint32_t nwg, uint32_t C, float eps, const float* __restrict__ GB, uint32_t gOff, uint32_t bOff,
-                                                     float* __restrict__ AB) {
+__global__ void __launch_bounds__(256) k_gn_finalize(const float4* PT, uint32_t nwg, uint32_t C, float eps, const float* GB, uint32_t gOff, uint32_t bOff,
+                                                     float* AB) {
   __shared__ Chan sh[8];
   const uint32_t g = blockIdx.x, t = threadIdx.x, l = t & 31u, cpg = C / 32u;
+  grid_dependency_wait();
+  grid_launch_dependents();
   Chan s{0.0f, 0.0f, 0.0f};
 #pragma unroll 4
-  for (uint32_t w = t; w < nwg; w += 256u) { const float4 q = __ldg(PT + (size_t)w * 32u + g); s = chan_merge(s, Chan{q.x, q.y, q.z}); }
+  for (uint32_t w = t; w < nwg; w += 256u) { const float4 q = ld_now(PT + (size_t)w * 32u + g); s = chan_merge(s, Chan{q.x, q.y, q.z}); }
 #pragma unroll
   for (uint32_t o = 1; o < 32u; o <<= 1) {
     Chan b; b.n = __shfl_xor_sync(0xffffffffu, s.n, o); b.mean = __shfl_xor_sync(0xffffffffu, s.mean, o); b.m2 = __shfl_xor_sync(0xffffffffu, s.m2, o);
@@ -127,8 +134,8 @@ __global__ void __launch_bounds__(256) k_gn_finalize(const float4* __restrict__ 
   for (int w = 1; w < 8; w++) s = chan_merge(s, sh[w]);
   const float rs = rsqrtf(s.m2 / fmaxf(s.n, 1.0f) + eps);
   const uint32_t c = g * cpg + t;
-  const float a = __ldg(GB + gOff + c) * rs;
-  AB[c] = a; AB[C + c] = __ldg(GB + bOff + c) - s.mean * a;
+  const float a = ld_now(GB + gOff + c) * rs;
+  AB[c] = a; AB[C + c] = ld_now(GB + bOff + c) - s.mean * a;
 }
 
 inline bool live(const p0p_ctx* c, const p0p_buf* b) { return b && c->bufs.count(const_cast<p0p_buf*>(b)); }
@@ -148,8 +155,7 @@ extern "C" int p0p_pixstats(p0p_ctx* c, const p0p_buf* x, uint64_t x_off, uint32
   const uint32_t vec = (C % 8u == 0u && ((uintptr_t)X & 15u) == 0u) ? 1u : 0u;
   uint32_t L = 1u; while (L < 32u && L * (vec ? 8u : 1u) < C) L <<= 1;                     // lanes per voxel: enough for one load each, at most a warp
   const uint64_t threads = (uint64_t)V * L;
-  k_pixstats<<<(unsigned)((threads + 255u) / 256u), 256, 0, c->stream>>>(X, V, C, L, eps != 0.0f ? eps : 1e-8f, (float*)r->ptr + ro, vec);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(k_pixstats, dim3((unsigned)((threads + 255u) / 256u)), dim3(256), 0, c->stream, X, V, C, L, eps != 0.0f ? eps : 1e-8f, (float*)r->ptr + ro, vec);
   if (e != cudaSuccess) return cuda_fail(c, e, "pixstats launch");
   c->launches += 1;
   return 0;
@@ -166,9 +172,8 @@ extern "C" int p0p_gn_partial(p0p_ctx* c, const p0p_buf* x, uint64_t x_off, uint
   const uint64_t xb = (uint64_t)pix * C * 2ull, pb = ((uint64_t)wgOff + nwg) * 512ull;
   if (x_off > x->size || xb > x->size - x_off || pb > part->size) return fail(c, -7, "gnPartial: a range is outside its buffer");
   DeviceGuard g(c->device);
-  (C == 32u ? k_gn_partial<1> : C == 64u ? k_gn_partial<2> : C == 128u ? k_gn_partial<4> : C == 256u ? k_gn_partial<8> : k_gn_partial<16>)
-      <<<nwg, 256, 0, c->stream>>>(reinterpret_cast<const __half*>((const char*)x->ptr + x_off), pix, wgOff, (float4*)part->ptr);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(C == 32u ? k_gn_partial<1> : C == 64u ? k_gn_partial<2> : C == 128u ? k_gn_partial<4> : C == 256u ? k_gn_partial<8> : k_gn_partial<16>,
+                                 dim3(nwg), dim3(256), 0, c->stream, reinterpret_cast<const __half*>((const char*)x->ptr + x_off), pix, wgOff, (float4*)part->ptr);
   if (e != cudaSuccess) return cuda_fail(c, e, "gnPartial launch");
   c->launches += 1;
   return 0;
@@ -182,8 +187,8 @@ extern "C" int p0p_gn_finalize(p0p_ctx* c, const p0p_buf* part, uint32_t nwg, ui
   if ((uint64_t)nwg * 512ull > part->size || ((uint64_t)std::max(g_off, b_off) + C) * 4ull > gb->size || ((uint64_t)ab_off + 2ull * C) * 4ull > ab->size)
     return fail(c, -7, "gnFinalize: a range is outside its buffer");
   DeviceGuard g(c->device);
-  k_gn_finalize<<<32, 256, 0, c->stream>>>((const float4*)part->ptr, nwg, C, eps != 0.0f ? eps : 1e-6f, (const float*)gb->ptr, g_off, b_off, (float*)ab->ptr + ab_off);
-  cudaError_t e = cudaGetLastError();
+  cudaError_t e = launch_chained(k_gn_finalize, dim3(32), dim3(256), 0, c->stream, (const float4*)part->ptr, nwg, C, eps != 0.0f ? eps : 1e-6f, (const float*)gb->ptr, g_off, b_off,
+                                 (float*)ab->ptr + ab_off);
   if (e != cudaSuccess) return cuda_fail(c, e, "gnFinalize launch");
   c->launches += 1;
   return 0;

@@ -54,6 +54,9 @@ __device__ __forceinline__ void cluster_sync() {
 // writes (the wait returns once that kernel has finished and its writes are visible; without the attribute it returns
 // at once).  grid_launch_dependents() tells the scheduler that the kernel after this one may begin to launch.
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// What it may overlap with must not be read through the read-only path (__ldg, const __restrict__): such loads may be moved above
+// the wait.  ld_now is a plain load.
+template <class T> __device__ __forceinline__ T ld_now(const T* p) { return *p; }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // global -> shared bulk copy; both addresses 16-byte aligned, bytes a multiple of 16; completes on `bar`

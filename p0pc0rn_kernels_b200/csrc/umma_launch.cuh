@@ -17,13 +17,15 @@ namespace p0p {
 // loads, the row's statistics and one 16-byte store.  (One thread per four elements, finding its row by a 64-bit division and
 // reading the vectors for every element: 17.4 us at 3600 rows of 3072 with LayerNorm + modulation, 12.7 now)
 template <bool LNMOD>
-__global__ void __launch_bounds__(128) k_prologue_f16(const KP p, __half* __restrict__ out) {
+__global__ void __launch_bounds__(128) k_prologue_f16(const KP p, __half* out) {
   const uint32_t k = (blockIdx.x * 128u + threadIdx.x) * 8u;
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (k >= p.K) return;
   const float* pv = p.PV + p.pvOff + p.kx0 + k;
   float g1[8], g2[8];
 #pragma unroll
-  for (int j = 0; j < 8; j++) { g1[j] = __ldg(pv + j); g2[j] = LNMOD ? __ldg(pv + p.pvStride + j) : 0.0f; }
+  for (int j = 0; j < 8; j++) { g1[j] = ld_now(pv + j); g2[j] = LNMOD ? ld_now(pv + p.pvStride + j) : 0.0f; }
   const float* x = reinterpret_cast<const float*>(p.X) + p.kx0 + k;
   auto row = [&](uint32_t m, const float4 a, const float4 b, float mean, float rstd) {
     const float xv[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
@@ -35,9 +37,9 @@ __global__ void __launch_bounds__(128) k_prologue_f16(const KP p, __half* __rest
   for (uint32_t m = blockIdx.y; m < p.M; m += 2u * gridDim.y) {
     const uint32_t n = min(m + gridDim.y, p.M - 1u);                  // the second row (a repeat of the last one past the end: not stored)
     const float4* xa = reinterpret_cast<const float4*>(x + (size_t)m * p.ldx); const float4* xb = reinterpret_cast<const float4*>(x + (size_t)n * p.ldx);
-    const float4 a0 = __ldg(xa), a1 = __ldg(xa + 1), b0 = __ldg(xb), b1 = __ldg(xb + 1);
+    const float4 a0 = ld_now(xa), a1 = ld_now(xa + 1), b0 = ld_now(xb), b1 = ld_now(xb + 1);
     const float* sa = p.ST + ((size_t)p.statOff + m) * 2u; const float* sb = p.ST + ((size_t)p.statOff + n) * 2u;
-    const float ma = __ldg(sa), ra = __ldg(sa + 1), mb = __ldg(sb), rb = __ldg(sb + 1);
+    const float ma = ld_now(sa), ra = ld_now(sa + 1), mb = ld_now(sb), rb = ld_now(sb + 1);
     row(m, a0, a1, ma, ra);
     if (m + gridDim.y < p.M) row(n, b0, b1, mb, rb);
   }
@@ -48,11 +50,13 @@ __global__ void __launch_bounds__(128) k_prologue_f16(const KP p, __half* __rest
 // tensor map's out-of-range fill), as the reference does.  Bound by the arithmetic of exp and division beside memory; a thread
 // (x = eight channels, y = pixel) keeps its channels' a and b in registers and walks the pixels, two in flight.
 // (One thread per eight elements, finding its channel by a 64-bit remainder: 20.2 us at 128 x 128 x 512, 15.4 now)
-__global__ void __launch_bounds__(256) k_prologue_gn(const KP p, __half* __restrict__ out) {
+__global__ void __launch_bounds__(256) k_prologue_gn(const KP p, __half* out) {
   const uint32_t c = (blockIdx.x * blockDim.x + threadIdx.x) * 8u, pix = p.Hi * p.Wi, step = gridDim.y * blockDim.y;
+  grid_dependency_wait();
+  grid_launch_dependents();
   float a[8], b[8];
 #pragma unroll
-  for (int j = 0; j < 8; j++) { a[j] = __ldg(p.PV + p.pvOff + c + j); b[j] = __ldg(p.PV + p.pvOff + p.pvStride + c + j); }
+  for (int j = 0; j < 8; j++) { a[j] = ld_now(p.PV + p.pvOff + c + j); b[j] = ld_now(p.PV + p.pvOff + p.pvStride + c + j); }
   const __half* x = reinterpret_cast<const __half*>(p.X) + c;
   auto apply = [&](uint32_t m, const uint4 q) {
     const __half* h = reinterpret_cast<const __half*>(&q);
@@ -63,7 +67,7 @@ __global__ void __launch_bounds__(256) k_prologue_gn(const KP p, __half* __restr
   };
   for (uint32_t m = blockIdx.y * blockDim.y + threadIdx.y; m < pix; m += 2u * step) {
     const uint32_t n = m + step;
-    const uint4 q0 = __ldg(reinterpret_cast<const uint4*>(x + (size_t)m * p.Ci)), q1 = __ldg(reinterpret_cast<const uint4*>(x + (size_t)min(n, pix - 1u) * p.Ci));
+    const uint4 q0 = ld_now(reinterpret_cast<const uint4*>(x + (size_t)m * p.Ci)), q1 = ld_now(reinterpret_cast<const uint4*>(x + (size_t)min(n, pix - 1u) * p.Ci));
     apply(m, q0);
     if (n < pix) apply(n, q1);
   }
@@ -310,8 +314,7 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   if (pre) {
     // about eight blocks per SM, but at least two rows to a thread where there are that many (the vectors are read once per thread)
     const uint32_t gx = (p.K / 8u + 127u) / 128u, gy = std::min(std::max(1u, 8u * sms / gx), (p.M + 1u) / 2u);
-    (p.xmode == P0P_X_LNMOD ? k_prologue_f16<true> : k_prologue_f16<false>)<<<dim3(gx, gy), 128, 0, c->stream>>>(p, reinterpret_cast<__half*>(c->scratch));
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(p.xmode == P0P_X_LNMOD ? k_prologue_f16<true> : k_prologue_f16<false>, dim3(gx, gy), dim3(128), 0, c->stream, p, reinterpret_cast<__half*>(c->scratch));
     if (e != cudaSuccess) return cuda_fail(c, e, "prologue launch");
     c->launches += 1;
     xbase = c->scratch;
@@ -319,8 +322,7 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
     // the block's x covers channels (Ci is a multiple of 64: eight, 16 or 32 threads of eight channels divide it), its y pixels
     const uint32_t oct = p.Ci / 8u, bx = oct % 32u == 0u ? 32u : oct % 16u == 0u ? 16u : 8u, by = 256u / bx, gx = oct / bx;
     const uint32_t gy = std::min(std::max(1u, 8u * sms / gx), (p.Hi * p.Wi + 2u * by - 1u) / (2u * by));
-    k_prologue_gn<<<dim3(gx, gy), dim3(bx, by), 0, c->stream>>>(p, reinterpret_cast<__half*>(c->scratch));
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(k_prologue_gn, dim3(gx, gy), dim3(bx, by), 0, c->stream, p, reinterpret_cast<__half*>(c->scratch));
     if (e != cudaSuccess) return cuda_fail(c, e, "GroupNorm prologue launch");
     c->launches += 1;
     xbase = c->scratch;
@@ -358,15 +360,15 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   const uint32_t plan[8] = {u.BT, u.KW, u.LOCK, u.NS, u.NA, u.NACC, u.S, u.T0};
   std::copy(plan, plan + 8, c->last_plan);
   void* args[3] = {&u, &mx, &mw};
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension; at[0].val.clusterDim.x = NB; at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cudaLaunchAttribute at[2];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;      // (see launch_chained)
+  at[1].id = cudaLaunchAttributeClusterDimension; at[1].val.clusterDim.x = NB; at[1].val.clusterDim.y = at[1].val.clusterDim.z = 1;
   cudaLaunchConfig_t cfg{};
-  cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(U_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = c->stream; cfg.attrs = at; cfg.numAttrs = pair ? 1u : 0u;
+  cfg.gridDim = dim3((unsigned)grid); cfg.blockDim = dim3(U_THREADS); cfg.dynamicSmemBytes = smem; cfg.stream = c->stream; cfg.attrs = at; cfg.numAttrs = pair ? 2u : 1u;
   if ((e = cudaLaunchKernelExC(&cfg, reinterpret_cast<const void*>(kern), args)) != cudaSuccess) return cuda_fail(c, e, "tensor-core kernel launch");
   c->launches += 1;
   if (u.S > 1u) {
-    void* fargs[1] = {&u};
-    if ((e = cudaLaunchKernel(reinterpret_cast<const void*>(umma_finish_kernel(p.epi)), dim3((tiles_all - u.T0) * NB, (BT + U_EPI_TB - 1u) / U_EPI_TB), dim3(128), fargs, 0, c->stream)) != cudaSuccess)
+    if ((e = launch_chained(umma_finish_kernel(p.epi), dim3((tiles_all - u.T0) * NB, (BT + U_EPI_TB - 1u) / U_EPI_TB), dim3(128), 0, c->stream, u)) != cudaSuccess)
       return cuda_fail(c, e, "split-K second stage launch");
     c->launches += 1;
   }
