@@ -164,11 +164,11 @@ extern "C" int p0p_gemm(p0p_ctx* c, const p0p_gemm_args* a_in, double* flops) {
   int rc = 0;
   // The streaming kernel wins up to 8 tokens (it never dequantises); from 9 on its second token group doubles its work and
   // the tensor-core kernel (narrow tiles, K-split accumulators, split-K) is faster on every shape measured.
-  // (5 to 8 tokens over a small weight, under 16 MB: the stream is too short to pay for the two launches and the split-K
-  // reduction; measured 14.7 against 19.3 us at 4096 x 4096.)
+  // (5 to 8 tokens over a weight of up to 40 MB: the stream is too short to pay for the split-K reduction.  Measured at 5 and 8
+  // tokens, decode / tensor cores: 4096 x 4096 13.0, 15.2 / 11.5 us; 4096 x 14336 19.4, 22.6 / 18.8; 28672 x 4096 23.6, 26.7 / 31.1.)
   const bool dec_ok = decode_supported(p), um_ok = umma_supported(c, p);
   const uint64_t stream_bytes = (uint64_t)N * K * (a->enc == P0P_ENC_Q4 ? 5u : 8u) / 8u;
-  const bool small_weight = p.M >= 5u && stream_bytes <= (16ull << 20);
+  const bool small_weight = p.M >= 5u && stream_bytes <= (40ull << 20);
   if (want == P0P_K_DECODE || (want == P0P_K_AUTO && dec_ok && ((p.M <= 8u && !small_weight) || !um_ok))) {
     if (!dec_ok) return fail(c, -9, "gemm: the decode kernel does not take this configuration");
     rc = launch_decode(c, p); used = P0P_K_DECODE;

@@ -8,7 +8,7 @@
 //            LLM block's shapes (896 units on 444 blocks) with a few blocks that had 3 units against 2.
 //            In each block one producer lane moves whole records from global to
 //            shared memory with bulk asynchronous copies (cp.async.bulk, mbarrier-tracked, a ring of stages);
-//            eight consumer warps: four row groups of 16 rows, two warps each that split a stage's records.
+//            eight consumer warps: four row groups of 16 rows, two warps each that take the stages in turn or share them (D_TURNS).
 //            Codes go to the tensor cores WITHOUT being dequantised.  A 4-bit code q is left where it sits and read as
 //            an fp16 SUBNORMAL: masked to bits 0..3 of a half it is q * 2^-24, masked to bits 4..7 it is 16 q * 2^-24
 //            (its token is staged pre-divided by 16), one AND per code pair and no offset to correct for.  An 8-bit
@@ -37,13 +37,20 @@
 
 namespace p0p {
 
-constexpr int D_CONSUMERS = 256;            // 8 warps: 4 row groups of 16 rows x 2 warps that split each stage's records
+constexpr int D_CONSUMERS = 256;            // 8 warps: 4 row groups of 16 rows x 2 warps that divide the stages (D_TURNS)
 constexpr int D_THREADS = D_CONSUMERS + 32; // + the producer warp
 constexpr int D_PER_SM = 3;                 // blocks an SM's registers hold (288 threads x 72): the plan relies on every block being resident
-constexpr int D_STAGES = 5;
+// How the two warps of a row group divide the stages: in turn, so that what a warp pays per stage beside its records (the barrier,
+// addresses, scales) is paid half as often; or a half of each, which is the faster form where the records outweigh that (4-bit
+// weights, 5 tokens and more: 8 x 28672 x 4096 26.7 us against 28.7 in turn).  In turn, with k-blocks of 4096 for one token:
+// 1 x 16384 x 16384 38.2 -> 33.6 us, 1 x 28672 x 4096 20.4 -> 17.2.
+template <int ENC, int MP> constexpr bool D_TURNS = ENC == P0P_ENC_Q8 || MP < 8;
+// Stages of the ring: in turn an EVEN number, so that a slot always belongs to the same one of the two warps.  (With an odd number a
+// warp meets a slot in every second of its phases only, and a wait by parity cannot tell a phase from the one two before it.)
+template <int ENC, int MP> constexpr int D_RING = D_TURNS<ENC, MP> ? 4 : 5;
 constexpr int D_STAGE_K = 256;              // k per stage: 8 q4 records (10240 B) or 4 q8 records (16896 B): one bulk copy each
 constexpr int D_STAGE_BYTES_Q4 = 10240, D_STAGE_BYTES_Q8 = 16896;
-constexpr int D_MAX_KC = 2048;              // largest k-block
+constexpr int D_MAX_KC = 4096;              // largest k-block
 constexpr int D_SMEM_MAX = 144 * 1024;      // dynamic shared memory ceiling of the stream kernel
 
 struct DecodeP {
@@ -293,6 +300,9 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
   const KP& p = d.p;
   constexpr uint32_t TOK_PAD = ENC == P0P_ENC_Q4 ? 64u : 16u;           // keeps the operand loads free of bank conflicts
   constexpr uint32_t GS = ENC == P0P_ENC_Q4 ? 32u : 64u;
+  constexpr bool TURNS = D_TURNS<ENC, MP>;
+  constexpr int D_STAGES = D_RING<ENC, MP>;
+  static_assert(!TURNS || D_STAGES % 2 == 0, "slots alternate between the two warps of a row group");
   const uint32_t tok_stride = d.KC * 2u + TOK_PAD;
   // layout: stages | token tile (M rows + one row of zeros) | C fragments | Sx pairs | pair-combine buffer | barriers
   unsigned char* stages = smem;
@@ -300,14 +310,14 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
   unsigned char* xs = stages + D_STAGES * D_STAGE_BYTES;
   constexpr int NF = MP < 8 ? 1 : MP / 8;                                                      // accumulator fragments per lane
   float* ctc = reinterpret_cast<float*>(xs + (((p.M + 1u) * tok_stride + 127u) & ~127u));       // [group][pair] float4 (-Ca, -Cb, -Ca, -Cb)
-  float* cts = ctc + (d.KC / GS) * (MP / 2) * 4u;                                              // [group][pair] float2 (Sx_a, Sx_b)   (q4 only)
+  float* cts = ctc + (ENC == P0P_ENC_Q4 ? 0u : (d.KC / GS) * (MP / 2) * 4u);                   // [group][pair] float2 (Sx_a, Sx_b)   (q4 only; the C fragments are q8's)
   float* comb = cts + (ENC == P0P_ENC_Q4 ? (d.KC / GS) * (MP / 2) * 2u : 0u);                  // [4 row groups][32 lanes][4 * NF]
   uint64_t* bars = reinterpret_cast<uint64_t*>(comb + 4u * 32u * (4 * NF));
   const uint32_t full0 = smem_u32(bars), empty0 = smem_u32(bars + D_STAGES);
 
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
   if (tid == 0) {
-    for (int s = 0; s < D_STAGES; s++) { mbar_init(full0 + 8u * s, 1); mbar_init(empty0 + 8u * s, D_CONSUMERS / 32); }
+    for (int s = 0; s < D_STAGES; s++) { mbar_init(full0 + 8u * s, 1); mbar_init(empty0 + 8u * s, TURNS ? D_CONSUMERS / 64 : D_CONSUMERS / 32); }
     fence_mbar_init();
   }
   // the row of zeros that token columns past M read
@@ -317,8 +327,9 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
 
   const uint32_t i0 = d_range(d, blockIdx.x), i1 = d_range(d, blockIdx.x + 1u);      // this block's stages
   constexpr uint32_t REC = ENC == P0P_ENC_Q4 ? 1280u : 4224u, REC_K = ENC == P0P_ENC_Q4 ? 32u : 64u;
+  constexpr uint32_t RPS = D_STAGE_K / REC_K;                           // records of a stage: 8 (4-bit weights) or 4
+  static_assert(RPS == (ENC == P0P_ENC_Q4 ? 8u : 4u), "the record loops below are written out");
   constexpr uint32_t STAGE_TX = (D_STAGE_K / REC_K) * REC;              // a k-block is a whole number of stages (K % 128 == 0)
-  constexpr uint32_t RPW = (D_STAGE_K / REC_K) / 2u;                    // records of a stage per consumer warp (two warps share 16 rows)
 
   if (warp == D_CONSUMERS / 32) {
     // ------------------------------------------------------------------ producer: one lane streams the records
@@ -344,22 +355,23 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
   // -------------------------------------------------------------------- consumers: warp = (half, row group)
   const uint32_t g = lane >> 2, t4 = lane & 3u, rg = warp & 3u, half = warp >> 2;
   const uint32_t rlo = rg * 16u + g;                                     // this lane's rows: rlo and rlo + 8
-  // shared-window addresses that stay fixed for the whole kernel (this warp's first record of a stage included)
-  const uint32_t code0 = smem_u32(stages) + half * RPW * REC + (ENC == P0P_ENC_Q4 ? rlo * 16u + t4 * 4u : rlo * 64u + t4 * 16u);
-  const uint32_t sm0 = smem_u32(stages) + half * RPW * REC + (ENC == P0P_ENC_Q4 ? 1024u + rlo * 4u : 4096u + rlo * 2u);
+  // shared-window addresses that stay fixed for the whole kernel
+  const uint32_t from = TURNS ? 0u : half * (RPS / 2u);                  // this warp's first record of a stage
+  const uint32_t code0 = smem_u32(stages) + from * REC + (ENC == P0P_ENC_Q4 ? rlo * 16u + t4 * 4u : rlo * 64u + t4 * 16u);
+  const uint32_t sm0 = smem_u32(stages) + from * REC + (ENC == P0P_ENC_Q4 ? 1024u + rlo * 4u : 4096u + rlo * 2u);
   // token columns past M read the row of zeros
-  const uint32_t xrow0 = smem_u32(xs) + min(g, p.M) * tok_stride + half * RPW * REC_K * 2u + (ENC == P0P_ENC_Q4 ? t4 * 16u : t4 * 32u);
-  const uint32_t xrow1 = smem_u32(xs) + min(g + 8u, p.M) * tok_stride + half * RPW * REC_K * 2u + (ENC == P0P_ENC_Q4 ? t4 * 16u : t4 * 32u);
+  const uint32_t xrow0 = smem_u32(xs) + min(g, p.M) * tok_stride + from * REC_K * 2u + (ENC == P0P_ENC_Q4 ? t4 * 16u : t4 * 32u);
+  const uint32_t xrow1 = smem_u32(xs) + min(g + 8u, p.M) * tok_stride + from * REC_K * 2u + (ENC == P0P_ENC_Q4 ? t4 * 16u : t4 * 32u);
   // this lane's token pair (2 t4, 2 t4 + 1); + 4 pairs for tokens 8..15.  With a single token every lane reads pair 0
   // (one address per warp instead of four)
   const uint32_t tp = p.M == 1u ? 0u : t4;
   // few tokens: this lane's accumulator columns 2 t4, 2 t4 + 1 belong to record slot `slot`; as an operand column, g = slot_b * MP + token
   constexpr uint32_t GC = MP < 8 ? 8 / MP : 1;
   const uint32_t slot = MP < 8 ? t4 / (uint32_t)(MP / 2) : 0u, slot_b = MP < 8 ? g / (uint32_t)MP : 0u;
-  const uint32_t x_off = half * RPW * REC_K * 2u + t4 * 16u, x_zero = smem_u32(xs) + p.M * tok_stride + x_off, x_own = smem_u32(xs) + min(g % (uint32_t)MP, p.M) * tok_stride + x_off;
-  const uint32_t cts_s = smem_u32(cts) + (half * RPW + slot) * (uint32_t)(MP / 2) * 8u + (t4 % (uint32_t)(MP / 2)) * 8u;
-  const uint32_t ctc_l = smem_u32(ctc) + (half * RPW * (MP / 2) + tp) * 16u;
-  const uint32_t cts_l = smem_u32(cts) + (half * RPW * (MP / 2) + tp) * 8u;
+  const uint32_t x_off = t4 * 16u, x_zero = smem_u32(xs) + p.M * tok_stride + x_off, x_own = smem_u32(xs) + min(g % (uint32_t)MP, p.M) * tok_stride + x_off;
+  const uint32_t cts_s = smem_u32(cts) + slot * (uint32_t)(MP / 2) * 8u + (t4 % (uint32_t)(MP / 2)) * 8u;
+  const uint32_t ctc_l = smem_u32(ctc) + (from * (MP / 2) + tp) * 16u;
+  const uint32_t cts_l = smem_u32(cts) + (from * (MP / 2) + tp) * 8u;
   float* comb_l = comb + (rg * 32u + lane) * (4 * NF);
   DLane L;
   L.MLO = 0x000f000fu; L.MHI = 0x00f000f0u; L.MAGIC = 0x64006400u;      // (masks live in registers: as immediates each AND would cost a constant load)
@@ -392,6 +404,7 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
       for (int i = 0; i < 4; i++) { tot[h][i] = 0.0f; tmn[h][i] = 0.0f; }
 
     for (uint32_t k = kfrom; ok && k < kto; k += D_STAGE_K) {
+      if (TURNS && (s & 1u) != half) { if (++s == D_STAGES) { s = 0; ph ^= 1u; } continue; }      // the row group's other warp takes this stage
       if (!mbar_wait(full0 + 8u * s, ph, d.status, 102)) { ok = false; break; }
       const uint32_t so = anchor(s * D_STAGE_BYTES), ko = anchor(k);
       const uint32_t ca = code0 + so, sa = sm0 + so;
@@ -403,17 +416,21 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
         for (uint32_t j = 0; j < GC; j++) xk[j] = (slot_b == j ? x_own : x_zero) + ko * 2u;
         d_recs_q4<MP, 0>(tot[0], tmn[0], ca, sas, xk, sk, L);
         if constexpr (MP == 4) d_recs_q4<MP, 2>(tot[0], tmn[0], ca, sas, xk, sk, L);
+        d_recs_q4<MP, 4>(tot[0], tmn[0], ca, sas, xk, sk, L);
+        if constexpr (MP == 4) d_recs_q4<MP, 6>(tot[0], tmn[0], ca, sas, xk, sk, L);
       } else if constexpr (ENC == P0P_ENC_Q4) {
         const uint32_t sk = cts_l + (ko / GS) * (MP / 2) * 8u;
-        static_assert(D_STAGE_K == 256, "four q4 records / two q8 records per consumer warp and stage");
         d_rec_q4<MP, 0>(tot, tmn, ca, sa, xk0, xk1, sk, L);
         d_rec_q4<MP, 1>(tot, tmn, ca, sa, xk0, xk1, sk, L);
         d_rec_q4<MP, 2>(tot, tmn, ca, sa, xk0, xk1, sk, L);
         d_rec_q4<MP, 3>(tot, tmn, ca, sa, xk0, xk1, sk, L);
+        static_assert(!TURNS, "half of the eight records of a stage");
       } else {
         const uint32_t ck = ctc_l + (ko / GS) * (MP / 2) * 16u;
         d_rec_q8<MP, 0>(tot, ca, sa, xk0, xk1, ck, L);
         d_rec_q8<MP, 1>(tot, ca, sa, xk0, xk1, ck, L);
+        d_rec_q8<MP, 2>(tot, ca, sa, xk0, xk1, ck, L);
+        d_rec_q8<MP, 3>(tot, ca, sa, xk0, xk1, ck, L);
       }
       __syncwarp();
       if (lane == 0) mbar_arrive(empty0 + 8u * s);
