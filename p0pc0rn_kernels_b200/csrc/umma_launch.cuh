@@ -114,6 +114,34 @@ inline uint32_t conv_tile_rows(const KP& p, bool atm) {
   return best;
 }
 
+// What a 64-k step of a tile costs on a busy GPU, in cycles: measured from the rounds and steps of whole calls (see the rule for pairs
+// in launch_umma).
+inline uint64_t umma_kstep(bool atm, bool pair, uint32_t bt) {
+  if (!pair) return atm ? (bt <= 128u ? 750u : std::max(13u * bt / 4u, 975u)) : 358u + 14u * bt / 5u;
+  if (bt > 256u) return (bt > 320u ? 31u : 33u) * bt / 10u;                      // two multiplies per 16 k
+  return atm ? std::max(620u, 190u + 11u * bt / 4u) : 190u + 31u * bt / 10u;
+}
+inline bool conv_pairs(uint32_t R, uint32_t Wo) { const uint32_t m = R * Wo > 256u ? 4u : 2u; return R % m == 0u && (R * Wo) % (16u * m) == 0u; }      // whole image rows to each block's share of each multiply, 32 tokens to a multiply
+// The 2-D convolution's tile: of the shapes that fit, the one with the least rounds x step.  The largest tile, which a convolution over
+// a clip takes whatever its chunks, leaves most SMs idle on small images, and the smallest one of 8-bit weights keeps them from pairs:
+// 3x3, 512 channels, fp16 weights, 64 x 64 37.3 -> 33.8 us, 32 x 32 to 256 channels 36.3 -> 30.7; 8-bit, 128 x 128 96.5 -> 68.5.
+// (Stride 1 only: strided loads bound the others, 160 x 96 at stride 2 took 34.3 us as before and 35.4 in narrower tiles.)
+inline uint32_t conv2d_tile_rows(const KP& p, bool atm, uint32_t nt, uint32_t sms) {
+  uint32_t best = conv_tile_rows(p, atm);
+  if (p.stride != 1u) return best;
+  uint64_t cost = ~0ull;
+  for (uint32_t R = p.Ho; R >= 1u; R--) {
+    const uint32_t bt = R * p.Wo;
+    if (bt > (atm ? 384u : 256u) || p.Ho % R || bt < 16u || R > 256u || p.M % bt) continue;
+    if (bt <= 256u ? bt % 16u != 0u : (R % 2u != 0u || bt % 32u != 0u)) continue;
+    const bool pair = nt >= 2u && sms % 2u == 0u && p.M > 160u && conv_pairs(R, p.Wo);
+    const uint64_t nb = pair ? 2u : 1u, tiles = (nt + nb - 1u) / nb * (p.M / bt), slots = sms / nb;
+    const uint64_t t = (tiles + slots - 1u) / slots * umma_kstep(atm, pair, bt);
+    if (t * 20u < cost * 19u) { cost = t; best = R; }                              // (5 % better than a larger one)
+  }
+  return best;
+}
+
 inline bool umma_supported(const p0p_ctx*, const KP& p) {
   if (!tmap_encoder()) return false;
   if (p.K % 64u) return false;
@@ -162,7 +190,7 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   const uint32_t bt_max = atm ? 384u : 256u, KSn = p.K / 64u;
   const uint64_t epi_tok = (p.epi == P0P_EPI_HEADS || p.epi == P0P_EPI_ONORMGATE) ? 150u : p.epi == P0P_EPI_SWIGLU ? 30u : 24u;      // cycles of epilogue per token of a tile
   uint32_t BT;
-  if (is_conv) { u.cvR = conv_tile_rows(p, atm); BT = u.cvR * p.Wo; }
+  if (is_conv) { u.cvR = p.xmode == P0P_X_CONV ? conv2d_tile_rows(p, atm, u.nt_all, sms) : conv_tile_rows(p, atm); BT = u.cvR * p.Wo; }
   else if (p.M <= 256u) BT = std::max(16u, (p.M + 15u) & ~15u);
   else {
     double best = 1e300; BT = 0;
@@ -223,15 +251,13 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   bool pair = false;
   if (u.nt_all >= 2u && sms % 2u == 0u && p.M > 160u) {
     if (is_conv) {
-      const uint32_t m = BT > 256u ? 4u : 2u;                                          // (whole image rows to each block's share of each multiply, 32 tokens to a multiply)
-      if (u.cvR % m == 0u && BT % (16u * m) == 0u) { pair = true; sp = split(2u, BT, atm ? std::max(620u, 190u + 11u * BT / 4u) : 190u + 31u * BT / 10u, BT > 192u && atm ? epi_tok * BT : 0u); }
+      if (conv_pairs(u.cvR, p.Wo)) { pair = true; sp = split(2u, BT, umma_kstep(atm, true, BT), BT > 192u && atm ? epi_tok * BT : 0u); }
     } else {
-      const uint64_t alone = BT <= 128u ? 750u : atm ? std::max<uint64_t>(13u * BT / 4u, 975u) : 358u + 14u * BT / 5u;
-      uint64_t best = split(1u, BT, alone, u.NACC == 1u ? epi_tok * BT : 0u).cost;
+      uint64_t best = split(1u, BT, BT <= 128u ? 750u : umma_kstep(atm, false, BT), u.NACC == 1u ? epi_tok * BT : 0u).cost;
       const uint32_t top = std::min(bt_max, p.M <= 256u ? (p.M + 31u) & ~31u : bt_max);
       for (uint32_t cand = top; cand >= std::min(top, 160u); cand -= 32u) {
         if (cand > 256u && cand % 64u) continue;
-        const uint64_t kstep = cand > 256u ? (cand > 320u ? 31u : 33u) * cand / 10u : atm ? std::max(620u, 190u + 11u * cand / 4u) : 190u + 31u * cand / 10u;
+        const uint64_t kstep = umma_kstep(atm, true, cand);
         const bool two = !atm || cand <= 192u;
         const uint64_t hidden = 17u * epi_tok * cand / 10u, exposed = !two ? epi_tok * cand : hidden > KSn * kstep ? hidden - KSn * kstep : 0u;
         const Split q = split(2u, cand, kstep, exposed);

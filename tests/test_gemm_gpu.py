@@ -338,6 +338,30 @@ def test_conv_tensor_core(gpu, oracle, case):
     CS.check(CS.run_gpu(gpu, CS.build(dict(case, kernel="generic"))), want, case["name"] + " (generic)")
 
 
+# tiles shared by two blocks (256 columns and more, whole rows to each block), with and without the norm's pre-pass, at one and two
+# multiplies per 16 k, an odd count of 128-column tiles; small images take narrow tiles; the video convolution's pairs
+CONV_PAIR = [
+    dict(name="pair conv3x3 c64 f16 odd tiles", enc="f16", M=32 * 32, N=384, K=9 * 64, x_elems=32 * 32 * 64, w_scale=0.03, epi="bias",
+         conv=dict(kind="conv", Hi=32, Wi=32, Ci=64, Ho=32, Wo=32, stride=1, padT=1, padL=1, ks=3, gn=True)),
+    dict(name="pair conv3x3 c64 q8", enc="q8", M=32 * 40, N=256, K=9 * 64, x_elems=32 * 40 * 64,
+         conv=dict(kind="conv", Hi=32, Wi=40, Ci=64, Ho=32, Wo=40, stride=1, padT=1, padL=1, ks=3)),
+    dict(name="pair conv1x1 stride 2 c128 q4", enc="q4", M=16 * 16, N=256, K=128, x_elems=32 * 32 * 128, epi="f32",
+         conv=dict(kind="conv", Hi=32, Wi=32, Ci=128, Ho=16, Wo=16, stride=2, padT=0, padL=0, ks=1)),
+    dict(name="narrow conv3x3 c64 f16, one row of 16", enc="f16", M=16 * 16, N=64, K=9 * 64, x_elems=16 * 16 * 64, w_scale=0.03,
+         conv=dict(kind="conv", Hi=16, Wi=16, Ci=64, Ho=16, Wo=16, stride=1, padT=1, padL=1, ks=3)),
+    dict(name="pair conv3 c64 f16", enc="f16", M=2 * 16 * 16, N=256, K=27 * 64, x_elems=2 * 16 * 16 * 64, w_scale=0.03, epi="bias",
+         conv=dict(kind="conv3", Hi=16, Wi=16, Ci=64, Ho=16, Wo=16, stride=2, padT=0, padL=0, ks=1)),
+]
+
+
+@pytest.mark.parametrize("case", CONV_PAIR, ids=lambda c: c["name"])
+def test_conv_pair_tiles(gpu, oracle, case):
+    h = CS.build(dict(case))
+    got = CS.run_gpu(gpu, h)
+    assert P()._lib.KERNEL_NAMES.get(gpu.lastKernel) == "umma"
+    CS.check(got, CS.run_oracle(h), case["name"])
+
+
 @pytest.mark.parametrize("case", EXTRA + CONV, ids=lambda c: c["name"])
 @pytest.mark.parametrize("kernel", KERNELS + ["umma"])
 def test_fused_variants(gpu, oracle, case, kernel):
