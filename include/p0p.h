@@ -201,8 +201,8 @@ int p0p_peer_barrier(p0p_ctx* ctx, p0p_buf* flags, p0p_buf* const* peer_flags, u
  * 'heads' projection.  Q [Hq][Lq][128] f16, K / V [Hkv][Lk][128] f16 head-major, O [Lq][ldo] f16 token-major at column h*128.
  * mode 0 none, 1 causal + valid length (key j visible to query i iff j <= min(i, nvalid-1)), 2 valid length (j < nvalid);
  * Hkv 0 = Hq, Lk 0 = Lq, ldo 0 = Hq*128, scale 0 = 1/sqrt(128), nvalid 0 = Lk.  *flops = 4*Lq*Lk*128*Hq (:192).
- * Calls with at least 128 queries per head run on the tensor-memory kernel (tcgen05), which first writes a transposed copy
- * of V into the context's scratch memory (sized on the first such call: not while recording a graph). */
+ * Calls with at least 128 queries per head run on the tensor-memory kernel (tcgen05); fewer split the keys over the SMs, with partial
+ * results in the context's scratch memory (sized on the first such call; one recorded before that runs unsplit). */
 typedef struct p0p_attn_args {
   uint32_t struct_size;
   uint32_t Hq, Hkv, Lq, Lk, ldo, mode, nvalid;

@@ -70,6 +70,7 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
   const uint32_t keys = a->mode == 0u ? Lk : a->mode == 1u ? std::min(Lk, std::min(Lq, nvalid)) : std::min(Lk, nvalid), nt = (keys + 63u) / 64u;
   const uint64_t units = (uint64_t)Hkv * rbs;
   uint32_t S = units >= 2u * sms || units > c->n_counters ? 1u : std::min<uint32_t>(nt, (uint32_t)(2u * sms / units));
+  if (S > 1u && !scratch_fits(c, units * S * 16u * wm * (512u + 8u))) S = 1u;      // recorded before it ran once: one block per unit needs no scratch
   p.tps = (nt + S - 1u) / S; p.S = S = (nt + p.tps - 1u) / p.tps;
   if (S > 1u) {
     const uint64_t slabs = units * S * 16u * wm;

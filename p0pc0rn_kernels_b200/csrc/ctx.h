@@ -79,6 +79,7 @@ struct DeviceGuard {
 #define P0P_ALIVE(ctx) do { if (!(ctx)) return -1; if ((ctx)->status) return ::p0p::fail((ctx), (ctx)->status, "GPU device lost: %s", (ctx)->err.c_str()); } while (0)
 
 int ensure_scratch(p0p_ctx* c, uint64_t bytes);
+bool scratch_fits(p0p_ctx* c, uint64_t bytes);      // false: while recording, and the scratch memory would have to grow
 
 // Launch as a programmatic dependent of whatever precedes in the stream: the kernel may start while that one drains, and sets itself
 // up meanwhile.  A kernel launched so calls grid_dependency_wait() before it touches what an earlier kernel may write, and

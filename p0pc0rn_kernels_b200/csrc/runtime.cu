@@ -339,6 +339,7 @@ static bool stream_is_capturing(p0p_ctx* c) {
   return st != cudaStreamCaptureStatusNone;
 }
 
+bool scratch_fits(p0p_ctx* c, uint64_t bytes) { return c->scratch_bytes >= bytes || !stream_is_capturing(c); }
 int ensure_scratch(p0p_ctx* c, uint64_t bytes) {
   if (c->scratch_bytes >= bytes) return 0;
   if (stream_is_capturing(c)) return fail(c, -11, "this call needs %llu bytes of scratch memory, which cannot be sized while recording: run it once before p0p_capture_begin", (unsigned long long)bytes);

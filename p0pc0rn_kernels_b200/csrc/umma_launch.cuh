@@ -333,6 +333,7 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
 #endif
   u.NQ = qstage ? (uint32_t)std::min<size_t>(std::min<size_t>(U_NQ_MAX, (q_cap + qstage - 1) / qstage), (227 * 1024 - fixed) / qstage) : 0u;
   if (qstage && u.NQ < 2u) return fail(c, -12, "gemm: no room for the record stages of this tile shape");
+  if (u.S > 1u && !scratch_fits(c, pro_bytes + (uint64_t)u.S * (tiles_all - u.T0) * NB * BT * 128u * 4u + 256)) { u.S = 1u; u.T0 = tiles_all; }      // recorded before it ran once: whole tiles need no scratch
   const uint64_t sk_bytes = u.S > 1u ? (uint64_t)u.S * (tiles_all - u.T0) * NB * BT * 128u * 4u : 0u;
   if (pro_bytes + sk_bytes) {
     if (int r = ensure_scratch(c, pro_bytes + sk_bytes + 256)) return r;

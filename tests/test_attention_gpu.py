@@ -117,3 +117,29 @@ def test_attention_split_keys(gpu, oracle, Hq, Hkv, Lq, Lk, mode, nvalid):
             assert np.abs(got - want).max() <= 2e-2 * np.abs(want).max()
     finally:
         for b in (qb, kb, vb, ob): gpu.free(b)
+
+
+def test_split_calls_recorded_first(gpu, oracle):
+    """recorded before the context has any scratch memory, calls that would split keys or k run unsplit instead of being refused"""
+    import p0pc0rn_kernels_b200 as P
+    O = oracle
+    Hq, Hkv, Lk, N, K, M = 8, 2, 1000, 256, 4096, 64
+    Q = O.round_f16(O.randn(Hq * 128, 21, 0.5)); Kt = O.round_f16(O.randn(Hkv * Lk * 128, 22, 0.5)); V = O.round_f16(O.randn(Hkv * Lk * 128, 23))
+    X = O.round_f16(O.randn(M * K, 24)); W = O.round_f16(O.randn(N * K, 25, 0.02))
+    own = P.createGpu({"device": 0})
+    qb, kb, vb, xb, wb = own.upload(P.toF16(Q)), own.upload(P.toF16(Kt)), own.upload(P.toF16(V)), own.upload(P.toF16(X)), own.upload(P.toF16(W))
+    ob, yb = own.buffer(Hq * 256), own.buffer(M * N * 4)
+
+    def calls():
+        P.attention(own, {"q": {"buf": qb}, "k": {"buf": kb}, "v": {"buf": vb}, "o": {"buf": ob}, "Lq": 1, "Lk": Lk, "Hq": Hq, "Hkv": Hkv, "mode": 0})
+        P.gemm(own, {"w": {"enc": "f16", "buf": wb, "off": 0, "rows": N, "cols": K}, "x": {"buf": xb}, "y": {"buf": yb}, "M": M, "N": N, "K": K, "epi": "f32"})
+    g = own.record(calls)
+    try:
+        g.launch()
+        got = P.fromF16(own.read(ob).view(np.uint16)); want = O.cpu_attn(Q, Kt, V, Hq=Hq, Hkv=Hkv, Lq=1, Lk=Lk, mode=0, nvalid=Lk)
+        assert np.abs(got - want).max() <= 2e-2 * np.abs(want).max()
+        y = own.read(yb).view(np.float32).reshape(M, N); ref = X.reshape(M, K).astype(np.float64) @ W.reshape(N, K).astype(np.float64).T
+        assert np.linalg.norm(y - ref) <= 1e-5 * np.linalg.norm(ref)
+    finally:
+        g.free()
+        for b in (qb, kb, vb, xb, wb, ob, yb): own.free(b)
