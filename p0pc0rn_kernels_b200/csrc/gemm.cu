@@ -163,7 +163,7 @@ extern "C" int p0p_gemm(p0p_ctx* c, const p0p_gemm_args* a_in, double* flops) {
   int want = (int)a->force_kernel, used = 0;
   int rc = 0;
   // The streaming kernel wins up to 8 tokens (it never dequantises); from 9 on its second token group doubles its work and
-  // the tensor-core kernel (narrow tiles, K-split accumulators, split-K) is faster on every shape measured.
+  // the tensor-core kernel (narrow tiles, split-K) is faster on every shape measured.
   // (5 to 8 tokens over a weight of up to 40 MB: the stream is too short to pay for the split-K reduction.  Measured at 5 and 8
   // tokens, decode / tensor cores: 4096 x 4096 13.0, 15.2 / 11.5 us; 4096 x 14336 19.4, 22.6 / 18.8; 28672 x 4096 23.6, 26.7 / 31.1.)
   const bool dec_ok = decode_supported(p), um_ok = umma_supported(c, p);

