@@ -84,7 +84,7 @@ bool scratch_fits(p0p_ctx* c, uint64_t bytes);      // false: while recording, a
 // Launch as a programmatic dependent of whatever precedes in the stream: the kernel may start while that one drains, and sets itself
 // up meanwhile.  A kernel launched so calls grid_dependency_wait() before it touches what an earlier kernel may write, and
 // grid_launch_dependents() only after that wait (so that the kernel after it never overlaps the one before it).  Worth one to two
-// microseconds at each boundary between kernels: LLM block at 16 tokens (5 kernels) 75 -> 64 us, at 512 tokens 200 -> 190, 32:8 heads 1000
+// microseconds at each boundary between kernels: LLM block at 16 tokens (5 kernels) 75 -> 72 us, at 512 tokens 200 -> 193, 32:8 heads 1000
 // causal tokens 23.6 -> 20.6, one query over 4000 keys 10.4 -> 8.9, GroupNorm + convolution (4 kernels) 102 -> 97.
 template <class... P, class... A>
 inline cudaError_t launch_chained(void (*k)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A... args) {

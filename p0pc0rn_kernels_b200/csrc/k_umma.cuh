@@ -213,8 +213,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
   if (warp == 0) {
     // ================================================================= producer of the token tiles (and fp16 weight tiles)
     if (lane == 0) {
-      // (the records of quantised weights stream from the start; tokens, fp16 weights and everything the epilogue touches wait for the
-      // kernel before this one)
+      // (everything this kernel reads may have been written by the kernel before it, weights included)
       grid_dependency_wait();
       grid_launch_dependents();
       Ring r(NS);
@@ -264,6 +263,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     // ================================================================= producer of the quantised records: runs ahead of
     // everything else by NQ stages (its only wait is for a free record stage)
     if (ENC != P0P_ENC_F16 && lane == 0) {
+      grid_dependency_wait();
       Ring q(NQ);
       bool ok = true;
       const uint32_t last = (p.Nw >> 6) - 1u;                  // record tiles past the weight's end do not exist: their columns are never stored
