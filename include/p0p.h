@@ -104,7 +104,8 @@ int p0p_host_free(p0p_ctx* ctx, void* p);
 /* The reference's Runner batches dispatches into one command buffer per submit (src/core/gpu.js:203-257) to keep
  * the GPU fed; the CUDA analogue is a graph.  Between begin and end, p0p_gemm / p0p_rowstats / p0p_copy /
  * p0p_clear calls are recorded instead of run; p0p_graph_launch replays them in stream order.  Run the same
- * calls once before recording (first calls size the library's scratch memory). */
+ * calls once before recording (first calls size the library's scratch memory).  Scratch memory that a recording
+ * uses is kept until p0p_close, so later calls that need more of it do not invalidate the recording. */
 typedef struct p0p_graph p0p_graph;
 int p0p_capture_begin(p0p_ctx* ctx);
 int p0p_capture_end(p0p_ctx* ctx, p0p_graph** out);

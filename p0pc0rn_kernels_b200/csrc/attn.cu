@@ -75,7 +75,7 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
   if (S > 1u) {
     const uint64_t slabs = units * S * 16u * wm;
     if (int rc = ensure_scratch(c, slabs * (512u + 8u))) return rc;
-    p.part = reinterpret_cast<float*>(c->scratch); p.part_ml = reinterpret_cast<float2*>((char*)c->scratch + slabs * 512u); p.count = c->counters;
+    p.part = reinterpret_cast<float*>(c->scratch.ptr); p.part_ml = reinterpret_cast<float2*>((char*)c->scratch.ptr + slabs * 512u); p.count = c->counters;
   }
   const auto kern = wm == 1u ? k_attn_split<1> : wm == 2u ? k_attn_split<2> : k_attn_split<4>;
   int rc = once[wm == 4u ? 3 : wm].run(c->device, [&] { return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM); });

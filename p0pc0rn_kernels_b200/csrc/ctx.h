@@ -10,6 +10,7 @@
 #include <vector>
 
 #include "../../include/p0p.h"
+#include "scratch.h"
 
 struct p0p_buf {
   void* ptr = nullptr;
@@ -36,9 +37,8 @@ struct p0p_ctx {
   int last_kernel = 0;
   uint32_t last_plan[8] = {};   // the tensor-core kernel's plan of the last call (p0p_last_plan)
   uint64_t launches = 0;
-  // split-K partial sums of the decode kernel (grown on demand, owned by the context)
-  void* scratch = nullptr;
-  uint64_t scratch_bytes = 0;
+  // partial sums and fp16 copies of normed tokens (grown on demand, owned by the context)
+  p0p::Scratch scratch;
   // arrival counters of kernels whose last block finishes the work of the others: all zero between launches (that block resets its own)
   uint32_t* counters = nullptr;
   uint32_t n_counters = 0;

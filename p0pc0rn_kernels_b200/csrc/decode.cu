@@ -107,7 +107,7 @@ int launch_decode(p0p_ctx* c, const KP& p) {
   DecodeLaunch L{};
   const uint64_t sbytes = plan_decode(d, L, c->prop.multiProcessorCount, (size_t)c->prop.sharedMemPerMultiprocessor);
   if (int r = ensure_scratch(c, sbytes + 256)) return r;
-  d.scratch = reinterpret_cast<float*>(c->scratch);
+  d.scratch = reinterpret_cast<float*>(c->scratch.ptr);
   d.status = c->dev_status;
   const uint32_t plan[8] = {d.G, d.T, d.KC, d.S, d.whole, d.units, d.tiles, 0u};
   std::copy(plan, plan + 8, c->last_plan);

@@ -77,7 +77,7 @@ int p0p_close(p0p_ctx* c) {
   for (p0p_buf* b : c->bufs) destroy_buf(c, b);
   c->bufs.clear();
   evict(c, 0);
-  if (c->scratch) cudaFree(c->scratch);
+  c->scratch.clear([](void* p) { cudaFree(p); });
   if (c->counters) cudaFree(c->counters);
   if (c->host_status) cudaFreeHost(c->host_status);
   for (void* p : c->pinned) cudaFreeHost(p);
@@ -339,15 +339,13 @@ static bool stream_is_capturing(p0p_ctx* c) {
   return st != cudaStreamCaptureStatusNone;
 }
 
-bool scratch_fits(p0p_ctx* c, uint64_t bytes) { return c->scratch_bytes >= bytes || !stream_is_capturing(c); }
+bool scratch_fits(p0p_ctx* c, uint64_t bytes) { return c->scratch.bytes >= bytes || !stream_is_capturing(c); }
 int ensure_scratch(p0p_ctx* c, uint64_t bytes) {
-  if (c->scratch_bytes >= bytes) return 0;
-  if (stream_is_capturing(c)) return fail(c, -11, "this call needs %llu bytes of scratch memory, which cannot be sized while recording: run it once before p0p_capture_begin", (unsigned long long)bytes);
-  if (c->scratch) { cudaStreamSynchronize(c->stream); cudaFree(c->scratch); c->scratch = nullptr; c->scratch_bytes = 0; }
-  uint64_t want = bytes < (8ull << 20) ? (8ull << 20) : (bytes + (1ull << 20) - 1) & ~((1ull << 20) - 1);
-  cudaError_t e = cudaMalloc(&c->scratch, want);
-  if (e != cudaSuccess) return cuda_fail(c, e, "split-K scratch");
-  c->scratch_bytes = want;
-  return 0;
+  const bool recording = !(c->scratch.recorded && c->scratch.bytes >= bytes) && stream_is_capturing(c);
+  if (c->scratch.bytes >= bytes) { c->scratch.recorded |= recording; return 0; }
+  if (recording) return fail(c, -11, "this call needs %llu bytes of scratch memory, which cannot be sized while recording: run it once before p0p_capture_begin", (unsigned long long)bytes);
+  const int e = c->scratch.grow(bytes, [](void** p, uint64_t n) { const cudaError_t r = cudaMalloc(p, n); if (r != cudaSuccess) (void)cudaGetLastError(); return (int)r; },
+                                [&](void* p) { cudaStreamSynchronize(c->stream); cudaFree(p); });
+  return e ? cuda_fail(c, (cudaError_t)e, "split-K scratch") : 0;
 }
 }  // namespace p0p

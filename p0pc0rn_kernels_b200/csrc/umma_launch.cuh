@@ -341,20 +341,20 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   if (pre) {
     // about eight blocks per SM, but at least two rows to a thread where there are that many (the vectors are read once per thread)
     const uint32_t gx = (p.K / 8u + 127u) / 128u, gy = std::min(std::max(1u, 8u * sms / gx), (p.M + 1u) / 2u);
-    cudaError_t e = launch_chained(p.xmode == P0P_X_LNMOD ? k_prologue_f16<true> : k_prologue_f16<false>, dim3(gx, gy), dim3(128), 0, c->stream, p, reinterpret_cast<__half*>(c->scratch));
+    cudaError_t e = launch_chained(p.xmode == P0P_X_LNMOD ? k_prologue_f16<true> : k_prologue_f16<false>, dim3(gx, gy), dim3(128), 0, c->stream, p, reinterpret_cast<__half*>(c->scratch.ptr));
     if (e != cudaSuccess) return cuda_fail(c, e, "prologue launch");
     c->launches += 1;
-    xbase = c->scratch;
+    xbase = c->scratch.ptr;
   } else if (pre_gn) {
     // the block's x covers channels (Ci is a multiple of 64: eight, 16 or 32 threads of eight channels divide it), its y pixels
     const uint32_t oct = p.Ci / 8u, bx = oct % 32u == 0u ? 32u : oct % 16u == 0u ? 16u : 8u, by = 256u / bx, gx = oct / bx;
     const uint32_t gy = std::min(std::max(1u, 8u * sms / gx), (p.Hi * p.Wi + 2u * by - 1u) / (2u * by));
-    cudaError_t e = launch_chained(k_prologue_gn, dim3(gx, gy), dim3(bx, by), 0, c->stream, p, reinterpret_cast<__half*>(c->scratch));
+    cudaError_t e = launch_chained(k_prologue_gn, dim3(gx, gy), dim3(bx, by), 0, c->stream, p, reinterpret_cast<__half*>(c->scratch.ptr));
     if (e != cudaSuccess) return cuda_fail(c, e, "GroupNorm prologue launch");
     c->launches += 1;
-    xbase = c->scratch;
+    xbase = c->scratch.ptr;
   }
-  u.sk_part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(c->scratch) + pro_bytes);
+  u.sk_part = reinterpret_cast<float*>(reinterpret_cast<unsigned char*>(c->scratch.ptr) + pro_bytes);
   {   // a wave of `sms` tiles reads G token tiles and sms / G weight tiles: least bytes at G = sqrt(sms * weight tile / token tile)
     const double wt = 128.0 * NB * (p.enc == P0P_ENC_Q4 ? 0.625 : p.enc == P0P_ENC_Q8 ? 1.03125 : 2.0), xt = 2.0 * BT;
     const double g = std::sqrt((double)slots * wt / xt);

@@ -623,6 +623,44 @@ def test_recorded_sequence(gpu, oracle):
         for b in bufs.values(): gpu.free(b)
 
 
+def test_recordings_outlive_the_scratch_they_used(gpu, oracle):
+    """recorded calls that keep partial results in scratch memory replay to the same bits after eager calls have outgrown that memory"""
+    O = oracle
+    Hq, Hkv, Lk, N, K, M = 32, 8, 4096, 256, 4096, 64
+    own = P().createGpu({"device": 0})
+    up = lambda a: own.upload(P().toF16(a))
+    q, k, v = up(O.randn(Hq * 128, 21, 0.5)), up(O.randn(Hkv * Lk * 128, 22, 0.5)), up(O.randn(Hkv * Lk * 128, 23))
+    x, w, o, y = up(O.randn(M * K, 24)), up(O.randn(N * K, 25, 0.02)), own.buffer(Hq * 256), own.buffer(M * N * 4)
+    big = 3000
+    xb, st, g, yb = own.upload(O.randn(big * K, 26)), own.buffer(big * 8), own.upload(np.ones(K, np.float32)), own.buffer(big * N * 4)
+    graphs, held = [], []
+
+    def calls():
+        P().attention(own, {"q": {"buf": q}, "k": {"buf": k}, "v": {"buf": v}, "o": {"buf": o}, "Lq": 1, "Lk": Lk, "Hq": Hq, "Hkv": Hkv, "mode": 2, "nvalid": 4000})
+        P().gemm(own, {"w": {"enc": "f16", "buf": w, "off": 0, "rows": N, "cols": K}, "x": {"buf": x}, "y": {"buf": y}, "M": M, "N": N, "K": K, "epi": "f32"})
+        assert own.lastPlan["S"] > 1, "the case must split"
+
+    def result(): return own.read(o).tobytes() + own.read(y).tobytes()
+    try:
+        calls()
+        want = result()
+        for rows in (1500, big):                                       # each needs more scratch than there is: 12, then 24 MB of fp16 tokens
+            graphs.append(own.record(calls))
+            P().rowstats(own, {"x": {"buf": xb}, "rows": rows, "cols": K, "mode": "rms", "eps": 1e-6, "st": {"buf": st}})
+            P().gemm(own, {"w": {"enc": "f16", "buf": w, "off": 0, "rows": N, "cols": K}, "x": {"buf": xb, "mode": "rms"}, "stats": {"buf": st}, "pv": {"buf": g},
+                           "y": {"buf": yb}, "M": rows, "N": N, "K": K, "epi": "f32"})
+            held.append(own.upload(np.full(8 << 20, 0x5A, np.uint8)))      # memory that a released block could have become
+            for gr in graphs:
+                own.upload(np.zeros(Hq * 128, np.uint16), "", o, 0); own.upload(np.zeros(M * N, np.float32), "", y, 0)
+                gr.launch()
+                assert result() == want
+            for b in held: assert (own.read(b) == 0x5A).all()
+    finally:
+        for gr in graphs: gr.free()
+        for b in (q, k, v, x, w, o, y, xb, st, g, yb, *held): own.free(b)
+        own.close()
+
+
 def test_rowstats(gpu, oracle):
     O = oracle
     rows, cols = 37, 1000
