@@ -623,6 +623,40 @@ def test_recorded_sequence(gpu, oracle):
         for b in bufs.values(): gpu.free(b)
 
 
+@pytest.mark.parametrize("M", [1, 4, 8, 16, 512])
+@pytest.mark.parametrize("enc", ["q4", "q8"])
+def test_weights_written_by_the_call_before(gpu, oracle, enc, M):
+    """a multiply whose encoded weight is the output of the launch directly before it: no kernel may read its weight before that launch
+    has finished.  The writer multiplies by the identity, so the fp16 values it stores are the weight's bytes."""
+    O = oracle
+    N, K = 1024, 4096
+    rng = np.random.default_rng(3)
+    if enc == "q4":                                                    # codes whose pairs of bytes are finite, positive fp16 values: every fourth one at most 6
+        q = rng.integers(0, 16, (N // 64, K // 32, 64, 32), dtype=np.uint8); q[..., 3::4] %= 7
+        sm = O.to_f16(np.stack([rng.uniform(0.002, 0.02, q.shape[:3]), -rng.uniform(0.02, 0.1, q.shape[:3])], -1).astype(np.float32).ravel()).view(np.uint8).reshape(*q.shape[:2], 256)
+        Wb = np.concatenate([(q[..., 0::2] | q[..., 1::2] << 4).reshape(*q.shape[:2], 1024), sm], 2).ravel()
+    else:
+        q = rng.integers(-128, 128, (N // 64, K // 64, 64, 64), dtype=np.int8); q[..., 1::2] = np.abs(q[..., 1::2] // 2) % 60 + 1
+        s = O.to_f16(rng.uniform(0.0005, 0.002, q.shape[:3]).astype(np.float32).ravel()).view(np.uint8).reshape(*q.shape[:2], 128)
+        Wb = np.concatenate([q.view(np.uint8).reshape(*q.shape[:2], 4096), s], 2).ravel()
+    rows = Wb.size // 512
+    X = O.randn(M * K, 6)
+    xb, eye, y = gpu.upload(P().toF16(X)), gpu.upload(P().toF16(np.eye(256, dtype=np.float32).ravel())), gpu.buffer(M * N * 4)
+    src, w = gpu.upload(Wb), gpu.buffer(Wb.size)
+    write = {"w": {"enc": "f16", "buf": eye, "off": 0, "rows": 256, "cols": 256}, "x": {"buf": src}, "y": {"buf": w}, "M": rows, "N": 256, "K": 256}
+    mul = {"w": {"enc": CS.ENC_NAMES[enc], "buf": w, "off": 0, "bytes": Wb.size, "rows": N, "cols": K}, "x": {"buf": xb}, "y": {"buf": y}, "M": M, "N": N, "K": K, "epi": "f32"}
+    try:
+        want = P().fromF16(P().toF16(X)).reshape(M, K).astype(np.float64) @ O.from_f16(O.dequant(CS.ENC_NAMES[enc], Wb, 0, N, K)[0]).reshape(N, K).astype(np.float64).T
+        for _ in range(3):
+            gpu.upload(np.zeros(Wb.size, np.uint8), "", w, 0)
+            P().gemm(gpu, write); P().gemm(gpu, mul)
+            assert np.array_equal(gpu.read(w), Wb), "the writer's own output"
+            got = gpu.read(y, 0, M * N * 4).view(np.float32).reshape(M, N)
+            assert np.linalg.norm(got - want) <= 1e-3 * np.linalg.norm(want)          # (the oracle's weights are rounded to fp16)
+    finally:
+        for b in (xb, eye, y, src, w): gpu.free(b)
+
+
 def test_recordings_outlive_the_scratch_they_used(gpu, oracle):
     """recorded calls that keep partial results in scratch memory replay to the same bits after eager calls have outgrown that memory"""
     O = oracle
