@@ -323,7 +323,6 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
   // the row of zeros that token columns past M read
   for (uint32_t i = tid; i < tok_stride / 16u; i += D_THREADS) reinterpret_cast<uint4*>(xs + (size_t)p.M * tok_stride)[i] = make_uint4(0, 0, 0, 0);
   __syncthreads();
-  grid_launch_dependents();                 // the second stage may be brought onto the SMs now; it waits for this grid to finish
 
   const uint32_t i0 = d_range(d, blockIdx.x), i1 = d_range(d, blockIdx.x + 1u);      // this block's stages
   constexpr uint32_t REC = ENC == P0P_ENC_Q4 ? 1280u : 4224u, REC_K = ENC == P0P_ENC_Q4 ? 32u : 64u;
@@ -385,6 +384,7 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
   bool ok = true;
   // tokens, statistics and the scratch buffer may still be in use by the kernel before this one in the stream
   grid_dependency_wait();
+  grid_launch_dependents();                 // the second stage may be brought onto the SMs now; it waits for this grid to finish
   // `ok` turns false when a bounded wait ran out: the warp then skips all work but still meets the others at
   // the named barriers below, so nobody is left waiting for it.
   for (uint32_t si = i0; si < i1;) {
