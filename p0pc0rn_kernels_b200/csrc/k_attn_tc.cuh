@@ -113,11 +113,12 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base)), 0);
 
+  // (every role, also those that only meet the loads at barriers: the limit of a bounded wait starts when the inputs exist)
+  grid_dependency_wait();
+  grid_launch_dependents();
   if (warp == 0) {
     // ================================================================= loads
     if (lane == 0) {
-      grid_dependency_wait();              // (the other roles only touch memory after what is loaded here)
-      grid_launch_dependents();
       mbar_expect_tx(q_full, hasB ? 2u * ATC_TILE : ATC_TILE);
       for (uint32_t t = 0; t < (hasB ? 2u : 1u); t++)
         for (uint32_t c = 0; c < 2u; c++) tma_load_3d(q_sm + t * ATC_TILE + c * 16384u, &mapQ, (int)(c * 64u), (int)(q0 + t * 128u), (int)h, q_full);

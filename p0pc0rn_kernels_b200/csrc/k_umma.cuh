@@ -207,15 +207,17 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base)), 0);
 
+  // Everything this kernel reads may have been written by the kernel before it, weights included, and what it writes may still be in
+  // use there.  Every role waits here, also those that only meet the others at barriers: the limit of a bounded wait starts to run when
+  // the inputs exist, however long the kernel before takes.
+  grid_dependency_wait();
+  grid_launch_dependents();
   const uint32_t tiles = u.n_tiles * u.m_tiles, KS = p.K / 64u, units = u.T0 + (tiles - u.T0) * u.S;
   constexpr bool swiglu = EPI == P0P_EPI_SWIGLU;
 
   if (warp == 0) {
     // ================================================================= producer of the token tiles (and fp16 weight tiles)
     if (lane == 0) {
-      // (everything this kernel reads may have been written by the kernel before it, weights included)
-      grid_dependency_wait();
-      grid_launch_dependents();
       Ring r(NS);
       bool ok = true;
       auto load2 = [&](uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar) { if (PAIR) tma_load_2d_pair(dst, m, x, y, bar); else tma_load_2d(dst, m, x, y, bar); };
@@ -261,9 +263,8 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     }
   } else if (warp == 6u + U_DEQ_WARPS) {
     // ================================================================= producer of the quantised records: runs ahead of
-    // everything else by NQ stages (its only wait is for a free record stage)
+    // everything else by NQ stages (in its loop it waits for nothing but a free record stage)
     if (ENC != P0P_ENC_F16 && lane == 0) {
-      grid_dependency_wait();
       Ring q(NQ);
       bool ok = true;
       const uint32_t last = (p.Nw >> 6) - 1u;                  // record tiles past the weight's end do not exist: their columns are never stored
@@ -346,7 +347,6 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     // ================================================================= epilogue (TMEM lanes 32*(warp%4) .. +31)
     const uint32_t q = warp & 3u, c = q * 32u + lane;
     uint32_t tl = 0, pass = 0;
-    grid_dependency_wait();
     bool ok = true;
     const bool vec = epilogue_vec_ok(p);
     auto acc_free = [&](uint32_t b) { if (PAIR) mbar_arrive_cluster(cluster_addr(acc_empty + 8u * b, 0u)); else mbar_arrive(acc_empty + 8u * b); };
