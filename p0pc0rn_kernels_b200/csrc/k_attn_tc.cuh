@@ -213,7 +213,9 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
         }
         float mts = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
         mine[(j & 1u) * 512u] = mts;
+        tc_fence_before();                   // this warp's reads of S end before its partner writes P over columns 32..63 of them
         bar_sync_named((int)pair_bar, 64);
+        tc_fence_after();
         mts = fmaxf(mts, other[(j & 1u) * 512u]) * sc;
         if (__any_sync(0xffffffffu, mts > m_used + 8.0f)) {
           // raise the reference maximum of the warp's rows (its partner has the same rows and decides alike); O and l are rescaled to it
