@@ -59,9 +59,6 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 template <class T> __device__ __forceinline__ T ld_now(const T* p) { return *p; }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-// asks for global memory to be brought into L2 (16-byte aligned, a multiple of 16 bytes): a hint, allowed before
-// grid_dependency_wait(), since what an earlier kernel still writes lands in L2 as well
-__device__ __forceinline__ void l2_prefetch(const void* src, uint32_t bytes) { asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(src), "r"(bytes) : "memory"); }
 // global -> shared bulk copy; both addresses 16-byte aligned, bytes a multiple of 16; completes on `bar`
 __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
   asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(dst), "l"(src), "r"(bytes), "r"(bar) : "memory");
