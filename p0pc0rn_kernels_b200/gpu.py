@@ -252,13 +252,15 @@ class Gpu:
 
     @property
     def lastPlan(self) -> dict:
-        """the tensor-core kernel's plan of the last call it served (a test convenience)"""
+        """how the last call was cut up (a test convenience; the words of p0p_last_plan)"""
         out = (C.c_uint32 * 8)()
         self._check(lib.p0p_last_plan(self._h, out))
         v = [int(x) for x in out]
         if self.lastKernel == 2:      # the decode kernel
             return dict(zip(("G", "T", "KC", "S", "whole", "units", "tiles"), v))
-        return dict(zip(("BT", "KW", "LOCK", "NS", "NA", "NACC", "S", "T0"), v))
+        plan = dict(zip(("BT", "KW", "LOCK", "NS", "NA", "NACC", "S", "T0"), v))
+        plan["PAIR"], plan["LOCK"] = plan["LOCK"] >> 1, plan["LOCK"] & 1
+        return plan
 
     @property
     def launches(self) -> int:

@@ -339,19 +339,29 @@ def test_conv_tensor_core(gpu, oracle, case):
 
 
 # tiles shared by two blocks (256 columns and more, whole rows to each block), with and without the norm's pre-pass, at one and two
-# multiplies per 16 k, an odd count of 128-column tiles; small images take narrow tiles; the video convolution's pairs
+# multiplies per 16 k, an odd count of 128-column tiles; small images take narrow tiles; the video convolution's pairs.  `plan` is
+# what the library must have chosen: the case covers that and nothing else.
 CONV_PAIR = [
-    dict(name="pair conv3x3 c64 f16 odd tiles", enc="f16", M=32 * 32, N=384, K=9 * 64, x_elems=32 * 32 * 64, w_scale=0.03, epi="bias",
+    dict(name="pair conv3x3 c64 f16 odd tiles", enc="f16", M=32 * 32, N=384, K=9 * 64, x_elems=32 * 32 * 64, w_scale=0.03, epi="bias", plan=dict(PAIR=1, BT=64),
          conv=dict(kind="conv", Hi=32, Wi=32, Ci=64, Ho=32, Wo=32, stride=1, padT=1, padL=1, ks=3, gn=True)),
-    dict(name="pair conv3x3 c64 q8", enc="q8", M=32 * 40, N=256, K=9 * 64, x_elems=32 * 40 * 64,
+    dict(name="pair conv3x3 c64 q8", enc="q8", M=32 * 40, N=256, K=9 * 64, x_elems=32 * 40 * 64, plan=dict(PAIR=1, BT=160),
          conv=dict(kind="conv", Hi=32, Wi=40, Ci=64, Ho=32, Wo=40, stride=1, padT=1, padL=1, ks=3)),
-    dict(name="pair conv1x1 stride 2 c128 q4", enc="q4", M=16 * 16, N=256, K=128, x_elems=32 * 32 * 128, epi="f32",
+    dict(name="pair conv1x1 stride 2 c128 q4", enc="q4", M=16 * 16, N=256, K=128, x_elems=32 * 32 * 128, epi="f32", plan=dict(PAIR=1, BT=128),
          conv=dict(kind="conv", Hi=32, Wi=32, Ci=128, Ho=16, Wo=16, stride=2, padT=0, padL=0, ks=1)),
-    dict(name="narrow conv3x3 c64 f16, one row of 16", enc="f16", M=16 * 16, N=64, K=9 * 64, x_elems=16 * 16 * 64, w_scale=0.03,
+    dict(name="narrow conv3x3 c64 f16, one row of 16", enc="f16", M=16 * 16, N=64, K=9 * 64, x_elems=16 * 16 * 64, w_scale=0.03, plan=dict(PAIR=0, BT=16),
          conv=dict(kind="conv", Hi=16, Wi=16, Ci=64, Ho=16, Wo=16, stride=1, padT=1, padL=1, ks=3)),
-    dict(name="pair conv3 c64 f16", enc="f16", M=2 * 16 * 16, N=256, K=27 * 64, x_elems=2 * 16 * 16 * 64, w_scale=0.03, epi="bias",
+    dict(name="pair conv3 c64 f16", enc="f16", M=2 * 16 * 16, N=256, K=27 * 64, x_elems=2 * 16 * 16 * 64, w_scale=0.03, epi="bias", plan=dict(PAIR=1, BT=256),
          conv=dict(kind="conv3", Hi=16, Wi=16, Ci=64, Ho=16, Wo=16, stride=2, padT=0, padL=0, ks=1)),
+    dict(name="pair conv3x3 c64 q4 odd tiles, two multiplies of 160", enc="q4", M=80 * 80, N=384, K=9 * 64, x_elems=80 * 80 * 64, epi="bias", plan=dict(PAIR=1, BT=320),
+         conv=dict(kind="conv", Hi=80, Wi=80, Ci=64, Ho=80, Wo=80, stride=1, padT=1, padL=1, ks=3)),
+    dict(name="pair conv3x3 c64 q8 gn odd tiles, two multiplies of 192", enc="q8", M=80 * 96, N=384, K=9 * 64, x_elems=80 * 96 * 64, epi="bias", plan=dict(PAIR=1, BT=384),
+         conv=dict(kind="conv", Hi=80, Wi=96, Ci=64, Ho=80, Wo=96, stride=1, padT=1, padL=1, ks=3, gn=True)),
 ]
+
+
+def planned(gpu, case):
+    got = {k: gpu.lastPlan[k] for k in case["plan"]}
+    assert got == case["plan"], (case["name"], gpu.lastPlan)
 
 
 @pytest.mark.parametrize("case", CONV_PAIR, ids=lambda c: c["name"])
@@ -359,6 +369,7 @@ def test_conv_pair_tiles(gpu, oracle, case):
     h = CS.build(dict(case))
     got = CS.run_gpu(gpu, h)
     assert P()._lib.KERNEL_NAMES.get(gpu.lastKernel) == "umma"
+    planned(gpu, case)
     CS.check(got, CS.run_oracle(h), case["name"])
 
 
@@ -430,19 +441,36 @@ def test_tensor_core_kernel(gpu, oracle, case):
         assert gpu.lastPlan["KW"] == 4 and gpu.lastPlan["S"] == 1, gpu.lastPlan
 
 
-# two blocks per tile: token counts around the steps of 32 and the one / two accumulator and one / two multiply edges, an odd count of
-# 128-column tiles (the last pair's second block has nothing to store) under each kind of epilogue, units of a split k loop
+def _heads(hq, hkv, M, off=0): return dict(Ltot=M + off, Hq=hq, Hkv=hkv, rowOff=off, eps=1e-6)
+
+
+# two blocks per tile, at every width the plan has (160 .. 384 tokens: one and two accumulators, one and two multiplies per 16 k), an odd
+# count of 128-column tiles (the last pair's second block has nothing to store) under each kind of epilogue, and units of a split k
+# loop: every tile's (T0 = 0) and only the last round's.  `plan` is what the library must have chosen on 148 SMs.
 PAIRS = [
-    dict(name="pair q4 M161", enc="q4", M=161, N=256, K=512),
-    dict(name="pair q8 M192 odd tiles", enc="q8", M=192, N=384, K=256),
-    dict(name="pair q4 M257 odd tiles f32", enc="q4", M=257, N=128 * 5, K=576, epi="f32"),
-    dict(name="pair q8 M224 ragged columns resadd", enc="q8", M=224, N=328, K=320, epi="resadd", w_rows=384),
-    dict(name="pair q4 M512 odd tiles rms+swiglu", enc="q4", M=512, N=2 * 64 * 7, K=1024, xmode="rms", epi="swiglu"),
-    dict(name="pair q8 M400 odd heads lnmod", enc="q8", M=400, N=128 * 9, K=512, xmode="lnmod", epi="heads", heads=dict(Ltot=410, Hq=5, Hkv=2, rowOff=10, eps=1e-6)),
-    dict(name="pair q4 M256 split k, odd tiles", enc="q4", M=256, N=128 * 3, K=4096, epi="resadd"),
-    dict(name="pair f16 M170 bias", enc="f16", M=170, N=256, K=64, epi="bias"),
-    dict(name="pair f16 M513 odd tiles, ring wrap", enc="f16", M=513, N=128 * 3, K=1600),
-    dict(name="pair q4 many tiles", enc="q4", M=1000, N=128 * 150, K=256),
+    dict(name="pair q4 M161", enc="q4", M=161, N=256, K=512, plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="pair q8 M192 odd tiles", enc="q8", M=192, N=384, K=256, plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="pair q4 M257 odd tiles f32", enc="q4", M=257, N=128 * 5, K=576, epi="f32", plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="pair q8 M224 ragged columns resadd", enc="q8", M=224, N=328, K=320, epi="resadd", w_rows=384, plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="pair q4 M512 odd tiles rms+swiglu", enc="q4", M=512, N=2 * 64 * 7, K=1024, xmode="rms", epi="swiglu", plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="alone q8 M400 odd heads lnmod", enc="q8", M=400, N=128 * 9, K=512, xmode="lnmod", epi="heads", heads=_heads(5, 2, 400, 10), plan=dict(PAIR=0, BT=208, S=1)),
+    dict(name="pair q8 M323 odd heads lnmod", enc="q8", M=323, N=128 * 3, K=576, xmode="lnmod", epi="heads", heads=_heads(1, 1, 323, 10), plan=dict(PAIR=1, BT=160, NACC=2, S=1)),
+    dict(name="pair q8 M232 odd heads, one accumulator", enc="q8", M=232, N=128 * 5, K=256, epi="heads", heads=_heads(3, 1, 232), plan=dict(PAIR=1, BT=224, NACC=1, S=1)),
+    dict(name="pair q4 M256 long k, odd tiles", enc="q4", M=256, N=128 * 3, K=4096, epi="resadd", plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="pair q4 M200 split k, odd tiles", enc="q4", M=200, N=128 * 3, K=8192, epi="resadd", plan=dict(PAIR=1, BT=160, S=3, T0=0)),
+    dict(name="pair q4 M196 split k, odd heads", enc="q4", M=196, N=128 * 3, K=1024, epi="heads", heads=_heads(1, 1, 196, 3), plan=dict(PAIR=1, BT=160, S=2, T0=0)),
+    dict(name="pair q8 M1045 last round split, odd heads", enc="q8", M=1045, N=128 * 29, K=512, epi="heads", heads=_heads(27, 1, 1045), plan=dict(PAIR=1, BT=160, S=2, T0=74)),
+    dict(name="pair q4 M641 last round split, odd heads, one accumulator", enc="q4", M=641, N=128 * 51, K=512, epi="heads", heads=_heads(49, 1, 641), plan=dict(PAIR=1, BT=224, S=2, T0=74)),
+    dict(name="pair q4 M321 odd tiles resadd", enc="q4", M=321, N=128 * 49, K=256, epi="resadd", plan=dict(PAIR=1, BT=192, NACC=2, S=1)),
+    dict(name="pair q4 M483 odd tiles", enc="q4", M=483, N=128 * 51, K=256, plan=dict(PAIR=1, BT=256, NACC=1, S=1)),
+    dict(name="pair q8 M1039 odd tiles bias, two multiplies of 160", enc="q8", M=1039, N=128 * 29, K=256, epi="bias", plan=dict(PAIR=1, BT=320, S=1)),
+    dict(name="pair q4 M711 odd tiles swiglu, two multiplies of 192", enc="q4", M=711, N=2 * 64 * 51, K=256, epi="swiglu", plan=dict(PAIR=1, BT=384, S=1)),
+    dict(name="pair q8 M734 odd heads, two multiplies of 192", enc="q8", M=734, N=128 * 51, K=256, epi="heads", heads=_heads(49, 1, 734), plan=dict(PAIR=1, BT=384, S=1)),
+    dict(name="alone f16 M170 bias", enc="f16", M=170, N=256, K=64, epi="bias", plan=dict(PAIR=0, BT=176, S=1)),
+    dict(name="pair f16 M208 bias", enc="f16", M=208, N=384, K=512, epi="bias", plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="pair f16 M513 odd tiles, ring wrap", enc="f16", M=513, N=128 * 3, K=1600, plan=dict(PAIR=1, BT=160, S=1)),
+    dict(name="pair f16 M484 odd tiles f32", enc="f16", M=484, N=128 * 39, K=512, epi="f32", plan=dict(PAIR=1, BT=192, S=1)),
+    dict(name="pair q4 many tiles", enc="q4", M=1000, N=128 * 150, K=256, plan=dict(PAIR=1, BT=256, S=1, T0=300)),
 ]
 
 
@@ -452,6 +480,7 @@ def test_pair_tiles(gpu, oracle, case):
     h = CS.build(dict(case))
     got = CS.run_gpu(gpu, h)
     assert gpu.lastKernel == K_UMMA
+    planned(gpu, case)
     CS.check(got, CS.run_oracle(h), case["name"])
 
 
