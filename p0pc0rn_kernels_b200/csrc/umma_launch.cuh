@@ -247,9 +247,10 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   // the tile takes two multiplies (above 256 tokens, steps of 64).  A pair's tiles up to 192 tokens have two accumulators, so the
   // next tile's multiplies hide the epilogue: what the head epilogue wants (150 cycles a token; q8, 3600 x 9216 x 3072 with it: 242 us
   // alone, 235 with 320 tokens, 214 with 192).  gate/up of the LLM block at 512 tokens: 111.5 alone, 101.2 as a pair of 256 tokens;
-  // fp16 16384 x 512 x 4608: 88 and 74.5.  A convolution's tile is given (bits must not depend on it): a pair wherever its rows split.
+  // fp16 16384 x 512 x 4608: 88 and 74.5.  A convolution's tile is given (bits must not depend on it): a pair wherever its rows split, and over a clip by the tokens
+  // of a frame, so that chunks of few frames and the whole clip run alike.
   bool pair = false;
-  if (u.nt_all >= 2u && sms % 2u == 0u && p.M > 160u) {
+  if (u.nt_all >= 2u && sms % 2u == 0u && (p.xmode == P0P_X_CONV3 ? p.Ho * p.Wo : p.M) > 160u) {
     if (is_conv) {
       if (conv_pairs(u.cvR, p.Wo)) { pair = true; sp = split(2u, BT, umma_kstep(atm, true, BT), BT > 192u && atm ? epi_tok * BT : 0u); }
     } else {

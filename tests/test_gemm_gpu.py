@@ -143,6 +143,11 @@ TC_CLIPS = [
     dict(name="384-token tiles (two multiplies per step), fp16 weights, bias", T=4, H=8, W=48, C=64, N=128, enc="f16", bias=True),
     dict(name="q4 weights (operand in tensor memory), 256 output channels", T=4, H=4, W=32, C=128, N=256, enc="q4"),
     dict(name="q8 weights, 320-token tiles", T=3, H=4, W=80, C=64, N=128, enc="q8"),
+    # frames of 128 tokens and 256 channels: one frame has too few tokens for pairs of blocks, the whole clip enough
+    dict(name="fp16 weights, 256 output channels, small frames", T=4, H=4, W=32, C=64, N=256, enc="f16", bias=True),
+    dict(name="q8 weights, 256 output channels, small frames", T=4, H=4, W=32, C=64, N=256, enc="q8"),
+    dict(name="fp16 weights, 384 output channels, pairs of blocks", T=3, H=8, W=32, C=64, N=384, enc="f16"),
+    dict(name="q8 weights, 384 output channels, pairs of blocks", T=3, H=12, W=16, C=64, N=384, enc="q8"),
 ]
 
 
@@ -164,6 +169,7 @@ def test_conv3_tensor_core(gpu, oracle, clip):
     ya, yb, yc, ring = gpu.buffer(n * 2), gpu.buffer(n * 2), gpu.buffer(n * 2), gpu.buffer(3 * fx * 2)
     bb = gpu.upload(bias) if bias is not None else None
     X16 = P().toF16(X)
+    plans = set()
 
     def run(x, y, t0, nf, padL=0, ks=1):
         a = {"w": {"enc": encn, "buf": wb, "off": 0, "bytes": wb._pf, "rows": N, "cols": K}, "x": x, "y": y, "M": nf * H * W, "N": N, "K": K,
@@ -171,6 +177,7 @@ def test_conv3_tensor_core(gpu, oracle, clip):
         if bb is not None: a["epi"] = "bias"; a["ev"] = {"buf": bb}
         P().gemm(gpu, a)
         assert P()._lib.KERNEL_NAMES.get(gpu.lastKernel) == "umma", "conv3 did not take the tensor-core kernel"
+        plans.add((gpu.lastPlan["PAIR"], gpu.lastPlan["BT"], gpu.lastPlan["KW"], gpu.lastPlan["S"]))
 
     try:
         run({"buf": xb}, {"buf": ya}, 0, T)
@@ -190,6 +197,8 @@ def test_conv3_tensor_core(gpu, oracle, clip):
         a, b, c = (gpu.read(y, 0, n * 2).view(np.uint16) for y in (ya, yb, yc))
         assert np.array_equal(a, b), "chunked conv3 DIFFERS from the whole clip"
         assert np.array_equal(a, c), "ring conv3 DIFFERS from the whole clip"
+        assert len(plans) == 1, f"chunks and the whole clip are cut up differently: {plans}"
+        if "pairs" in clip["name"]: assert gpu.lastPlan["PAIR"] == 1
     finally:
         for x in (xb, wb, ya, yb, yc, ring, bb):
             if x is not None: gpu.free(x)
