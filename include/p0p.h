@@ -104,7 +104,9 @@ int p0p_host_free(p0p_ctx* ctx, void* p);
 /* The reference's Runner batches dispatches into one command buffer per submit (src/core/gpu.js:203-257) to keep
  * the GPU fed; the CUDA analogue is a graph.  Between begin and end, p0p_gemm / p0p_rowstats / p0p_copy /
  * p0p_clear calls are recorded instead of run; p0p_graph_launch replays them in stream order.  Run the same
- * calls once before recording (first calls size the library's scratch memory).  Scratch memory that a recording
+ * calls once before recording: first calls size the library's scratch memory, and a call that needs more of it than there is
+ * returns -11 while recording.  (Two kinds of call do without and run unsplit, slower and with sums in another order: attention
+ * of few queries, and a multiply that only the two-blocks-per-tile plan splits.  p0p_last_plan shows it.)  Scratch memory that a recording
  * uses is kept until p0p_close, so later calls that need more of it do not invalidate the recording. */
 typedef struct p0p_graph p0p_graph;
 int p0p_capture_begin(p0p_ctx* ctx);
@@ -154,7 +156,8 @@ uint64_t p0p_launch_count(const p0p_ctx* ctx);
  * tell which variant they covered.  out8 = {tokens per tile, k-steps of 64 k per pipeline step, bit 0 lock-step rings and
  * bit 1 two blocks per tile, token stages, operand stages, accumulator buffers, split-K units per tile, tiles left unsplit}.
  * After a call the decode kernel served: {blocks, stages of 256 k in the call, k-block length, k-blocks, 1 if the blocks' ranges are whole units, units, 64-row
- * tiles, 0}. */
+ * tiles, 0}.  After p0p_attention: {splits of the keys, key tiles of 64 per split, row tiles of 16 per block, row blocks per kv head} or,
+ * on the tensor-memory kernel, {two-tile blocks, one-tile blocks per head}. */
 int p0p_last_plan(const p0p_ctx* ctx, uint32_t* out8);
 
 /* No counterpart in the reference (a browser page never manages device memory).  The decode-sized q4 multiply

@@ -61,6 +61,8 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
     if (e != cudaSuccess) return cuda_fail(c, e, "attention launch");
     c->launches += 1;
     c->last_kernel = P0P_K_ATTN_TMEM;
+    const uint32_t plan[8] = {t.np, t.ns};
+    std::copy(plan, plan + 8, c->last_plan);
     return 0;
   }
   // ---- split-key kernel.  Row tiles per block: as few as hold the rows that share a kv head (fewer rows leave more warps to the
@@ -85,5 +87,7 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
   if (e != cudaSuccess) return cuda_fail(c, e, "attention launch");
   c->launches += 1;
   c->last_kernel = P0P_K_ATTN_WARP;
+  const uint32_t plan[8] = {p.S, p.tps, wm, rbs};
+  std::copy(plan, plan + 8, c->last_plan);
   return 0;
 }

@@ -249,6 +249,7 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
   // alone, 235 with 320 tokens, 214 with 192).  gate/up of the LLM block at 512 tokens: 111.5 alone, 101.2 as a pair of 256 tokens;
   // fp16 16384 x 512 x 4608: 88 and 74.5.  A convolution's tile is given (bits must not depend on it): a pair wherever its rows split, and over a clip by the tokens
   // of a frame, so that chunks of few frames and the whole clip run alike.
+  const bool alone_splits = sp.S > 1u;
   bool pair = false;
   if (u.nt_all >= 2u && sms % 2u == 0u && (p.xmode == P0P_X_CONV3 ? p.Ho * p.Wo : p.M) > 160u) {
     if (is_conv) {
@@ -334,7 +335,10 @@ inline int launch_umma(p0p_ctx* c, const KP& p0) {
 #endif
   u.NQ = qstage ? (uint32_t)std::min<size_t>(std::min<size_t>(U_NQ_MAX, (q_cap + qstage - 1) / qstage), (227 * 1024 - fixed) / qstage) : 0u;
   if (qstage && u.NQ < 2u) return fail(c, -12, "gemm: no room for the record stages of this tile shape");
-  if (u.S > 1u && !scratch_fits(c, pro_bytes + (uint64_t)u.S * (tiles_all - u.T0) * NB * BT * 128u * 4u + 256)) { u.S = 1u; u.T0 = tiles_all; }      // recorded before it ran once: whole tiles need no scratch
+  // Recorded before it ran once, without scratch memory for its partial sums: a call that splits as lone blocks too is refused below
+  // (-11: run it once, then record), like every call that needs more scratch than there is; one that only its pairs split runs
+  // whole tiles, which need none.
+  if (u.S > 1u && !alone_splits && !scratch_fits(c, pro_bytes + (uint64_t)u.S * (tiles_all - u.T0) * NB * BT * 128u * 4u + 256)) { u.S = 1u; u.T0 = tiles_all; }
   const uint64_t sk_bytes = u.S > 1u ? (uint64_t)u.S * (tiles_all - u.T0) * NB * BT * 128u * 4u : 0u;
   if (pro_bytes + sk_bytes) {
     if (int r = ensure_scratch(c, pro_bytes + sk_bytes + 256)) return r;

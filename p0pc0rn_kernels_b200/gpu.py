@@ -258,6 +258,8 @@ class Gpu:
         v = [int(x) for x in out]
         if self.lastKernel == 2:      # the decode kernel
             return dict(zip(("G", "T", "KC", "S", "whole", "units", "tiles"), v))
+        if self.lastKernel == 16: return dict(zip(("S", "tps", "row_tiles", "row_blocks"), v))      # attention, split keys
+        if self.lastKernel == 17: return dict(zip(("np", "ns"), v))                                 # attention, tensor memory
         plan = dict(zip(("BT", "KW", "LOCK", "NS", "NA", "NACC", "S", "T0"), v))
         plan["PAIR"], plan["LOCK"] = plan["LOCK"] >> 1, plan["LOCK"] & 1
         return plan

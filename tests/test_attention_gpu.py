@@ -120,7 +120,8 @@ def test_attention_split_keys(gpu, oracle, Hq, Hkv, Lq, Lk, mode, nvalid):
 
 
 def test_split_calls_recorded_first(gpu, oracle):
-    """recorded before the context has any scratch memory, calls that would split keys or k run unsplit instead of being refused"""
+    """recorded before the context has any scratch memory: attention that would split its keys runs unsplit (and says so), a multiply that
+    splits k is refused, and after one eager call both record as they run eagerly"""
     import p0pc0rn_kernels_b200 as P
     O = oracle
     Hq, Hkv, Lk, N, K, M = 8, 2, 1000, 256, 4096, 64
@@ -129,17 +130,38 @@ def test_split_calls_recorded_first(gpu, oracle):
     own = P.createGpu({"device": 0})
     qb, kb, vb, xb, wb = own.upload(P.toF16(Q)), own.upload(P.toF16(Kt)), own.upload(P.toF16(V)), own.upload(P.toF16(X)), own.upload(P.toF16(W))
     ob, yb = own.buffer(Hq * 256), own.buffer(M * N * 4)
+    plans = []
 
-    def calls():
+    def attn():
         P.attention(own, {"q": {"buf": qb}, "k": {"buf": kb}, "v": {"buf": vb}, "o": {"buf": ob}, "Lq": 1, "Lk": Lk, "Hq": Hq, "Hkv": Hkv, "mode": 0})
+        plans.append(own.lastPlan["S"])
+
+    def mul():
         P.gemm(own, {"w": {"enc": "f16", "buf": wb, "off": 0, "rows": N, "cols": K}, "x": {"buf": xb}, "y": {"buf": yb}, "M": M, "N": N, "K": K, "epi": "f32"})
-    g = own.record(calls)
-    try:
-        g.launch()
+        plans.append(own.lastPlan["S"])
+
+    def check():
         got = P.fromF16(own.read(ob).view(np.uint16)); want = O.cpu_attn(Q, Kt, V, Hq=Hq, Hkv=Hkv, Lq=1, Lk=Lk, mode=0, nvalid=Lk)
         assert np.abs(got - want).max() <= 2e-2 * np.abs(want).max()
+    graphs = []
+    try:
+        graphs.append(own.record(attn)); graphs[0].launch()
+        check()
+        assert plans == [1]
+        with pytest.raises(ValueError, match="run it once before"):
+            own.record(mul)
+        assert not own.lost
+        attn(); mul()
+        eager = own.read(ob).tobytes() + own.read(yb).tobytes()
+        graphs.append(own.record(lambda: (attn(), mul())))
+        assert plans[1:3] == plans[3:] and min(plans[1:3]) > 1, plans
+        own.upload(np.zeros(Hq * 128, np.uint16), "", ob, 0); own.upload(np.zeros(M * N, np.float32), "", yb, 0)
+        graphs[1].launch()
+        assert own.read(ob).tobytes() + own.read(yb).tobytes() == eager
+        check()
         y = own.read(yb).view(np.float32).reshape(M, N); ref = X.reshape(M, K).astype(np.float64) @ W.reshape(N, K).astype(np.float64).T
         assert np.linalg.norm(y - ref) <= 1e-5 * np.linalg.norm(ref)
     finally:
-        g.free()
+        for g in graphs: g.free()
         for b in (qb, kb, vb, xb, wb, ob, yb): own.free(b)
+        own.close()
