@@ -82,8 +82,8 @@ extern "C" int p0p_attention(p0p_ctx* c, const p0p_attn_args* a, double* flops) 
   const auto kern = wm == 1u ? k_attn_split<1> : wm == 2u ? k_attn_split<2> : k_attn_split<4>;
   int rc = once[wm == 4u ? 3 : wm].run(c->device, [&] { return (int)cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)AT_SMEM); });
   if (rc) return cuda_fail(c, (cudaError_t)rc, "attention kernel attribute");
-  if (Hkv > 65535u || rbs > 65535u) return fail(c, -5, "attention: at most 65535 kv heads and 65535 blocks of query rows");
-  cudaError_t e = launch_chained(kern, dim3(S, Hkv, rbs), dim3(128), AT_SMEM, c->stream, p);
+  if (Hkv > 65535u) return fail(c, -5, "attention: at most 65535 kv heads");
+  cudaError_t e = launch_chained(kern, dim3(rbs, Hkv, S), dim3(128), AT_SMEM, c->stream, p);
   if (e != cudaSuccess) return cuda_fail(c, e, "attention launch");
   c->launches += 1;
   c->last_kernel = P0P_K_ATTN_WARP;

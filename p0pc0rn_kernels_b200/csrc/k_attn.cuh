@@ -59,7 +59,7 @@ __global__ void __launch_bounds__(128) k_attn_split(const AttnP p) {
   __shared__ float sm_m[4][16], sm_l[4][16];
   __shared__ uint32_t sm_last;
   const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u, g = lane >> 2, t4 = lane & 3u, wm = warp % WM, wk = warp / WM;
-  const uint32_t split = blockIdx.x, hk = blockIdx.y, rb = blockIdx.z, r0 = rb * RB, grp = p.Hq / p.Hkv;
+  const uint32_t rb = blockIdx.x, hk = blockIdx.y, split = blockIdx.z, r0 = rb * RB, grp = p.Hq / p.Hkv;
   const __half* Kg = p.K + (size_t)hk * p.Lk * 128u; const __half* Vg = p.V + (size_t)hk * p.Lk * 128u;
   const __half* Qg = p.Q + (size_t)hk * grp * p.Lq * 128u;
   const uint32_t base = (uint32_t)__cvta_generic_to_shared(at_smem);
@@ -179,7 +179,7 @@ __global__ void __launch_bounds__(128) k_attn_split(const AttnP p) {
     __half2* d = reinterpret_cast<__half2*>(p.O + (size_t)i * p.ldo + h * 128u + 4u * lane);
     d[0] = __floats2half2_rn(v.x, v.y); d[1] = __floats2half2_rn(v.z, v.w);
   };
-  const size_t slab = ((size_t)hk * gridDim.z + rb) * p.S;
+  const size_t slab = ((size_t)hk * gridDim.x + rb) * p.S;
   for (uint32_t r = warp; r < nrows; r += 4u) {
     const uint32_t w0 = r >> 4, rr = r & 15u;
     float M = -INFINITY, L = 0.0f;
@@ -205,7 +205,7 @@ __global__ void __launch_bounds__(128) k_attn_split(const AttnP p) {
   __threadfence();
   __syncthreads();
   if (tid == 0u) {
-    uint32_t* c = p.count + hk * gridDim.z + rb;
+    uint32_t* c = p.count + hk * gridDim.x + rb;
     const uint32_t last = atomicAdd(c, 1u) == p.S - 1u ? 1u : 0u;
     if (last) *c = 0u;
     sm_last = last;

@@ -119,6 +119,31 @@ def test_attention_split_keys(gpu, oracle, Hq, Hkv, Lq, Lk, mode, nvalid):
         for b in (qb, kb, vb, ob): gpu.free(b)
 
 
+def test_attention_split_keys_many_row_blocks(gpu):
+    """more blocks of 64 query rows than a grid has in y or z (forced: the library's own choice for so many queries is the other kernel)"""
+    import torch
+
+    import p0pc0rn_kernels_b200 as P
+    Lq, Lk = 64 * 65536 + 5, 65
+    g = torch.Generator(device="cuda"); g.manual_seed(1)
+    q, k, v = (torch.empty(n, 128, device="cuda", dtype=torch.float16).normal_(0, 0.5, generator=g) for n in (Lq, Lk, Lk))
+    o = torch.full((Lq, 128), float("nan"), device="cuda", dtype=torch.float16)
+    torch.cuda.synchronize()
+    bufs = [gpu.wrap(t.data_ptr(), t.numel() * 2) for t in (q, k, v, o)]
+    try:
+        P.attention(gpu, {**{n: {"buf": b} for n, b in zip("qkvo", bufs)}, "Lq": Lq, "Lk": Lk, "Hq": 1, "mode": 0, "kernel": "warp"})
+        gpu.done()
+        assert gpu.lastPlan["row_blocks"] == 65537
+        for r0 in (0, 64 * 32767, 64 * 65535, Lq - 69):
+            want = torch.softmax(q[r0:r0 + 69].float() @ k.float().T / 128 ** 0.5, -1) @ v.float()
+            assert (o[r0:r0 + 69].float() - want).abs().max() <= 2e-2 * want.abs().max()
+        assert torch.isfinite(o).all()
+    finally:
+        for b in bufs: gpu.free(b)
+        del q, k, v, o
+        torch.cuda.empty_cache()
+
+
 def test_split_calls_recorded_first(gpu, oracle):
     """recorded before the context has any scratch memory: attention that would split its keys runs unsplit (and says so), a multiply that
     splits k is refused, and after one eager call both record as they run eagerly"""
