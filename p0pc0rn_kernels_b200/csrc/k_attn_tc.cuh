@@ -113,12 +113,13 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
   tc_fence_after();
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base)), 0);
 
-  // (every role, also those that only meet the loads at barriers: the limit of a bounded wait starts when the inputs exist)
-  grid_dependency_wait();
-  grid_launch_dependents();
+  // (every role waits for the kernel before, also those that only meet the loads at barriers: the limit of a bounded wait starts when the
+  // inputs exist)
   if (warp == 0) {
     // ================================================================= loads
     if (lane == 0) {
+      grid_dependency_wait();
+      grid_launch_dependents();
       mbar_expect_tx(q_full, hasB ? 2u * ATC_TILE : ATC_TILE);
       for (uint32_t t = 0; t < (hasB ? 2u : 1u); t++)
         for (uint32_t c = 0; c < 2u; c++) tma_load_3d(q_sm + t * ATC_TILE + c * 16384u, &mapQ, (int)(c * 64u), (int)(q0 + t * 128u), (int)h, q_full);
@@ -134,6 +135,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
     // ================================================================= multiplies (the whole warp walks the loop, one lane issues)
     const uint32_t idesc = umma_idesc_f16(128u, 128u), idesc_v = idesc | UMMA_B_MN, nt = hasB ? 2u : 1u;
     const uint64_t qd[2] = {umma_desc_sw128(q_sm), umma_desc_sw128(q_sm + ATC_TILE)};
+    grid_dependency_wait();
     bool ok = __all_sync(0xffffffffu, mbar_wait(q_full, 0u, p.status, 402) && mbar_wait(kv_full, 0u, p.status, 403));
     if (ok) {
       tc_fence_after();
@@ -192,6 +194,7 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
       const float sc = p.scale_log2;
       float m_used = -INFINITY, l = 0.0f;
       bool ok = true;
+      grid_dependency_wait();
       for (uint32_t j = 0; j < nj; j++) {
         // (a wait that ran out: the thread goes on without it, so that its partner is not left at the barrier; the status word is set)
         if (ok && !mbar_spin(s_full + 8u * t, j & 1u, p.status, 407)) ok = false;

@@ -208,10 +208,9 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
   const uint32_t tmem_base = __shfl_sync(0xffffffffu, *reinterpret_cast<volatile uint32_t*>(gbase + (tmem_slot - base)), 0);
 
   // Everything this kernel reads may have been written by the kernel before it, weights included, and what it writes may still be in
-  // use there.  Every role waits here, also those that only meet the others at barriers: the limit of a bounded wait starts to run when
-  // the inputs exist, however long the kernel before takes.
-  grid_dependency_wait();
-  grid_launch_dependents();
+  // use there.  Every role waits for it, also those that only meet the others at barriers: the limit of a bounded wait starts to run
+  // when the inputs exist, however long the kernel before takes.  Each waits where its own set-up ends (all of them at this point
+  // instead: LLM block at 16 tokens 72.5 us against 71.5, at 512 tokens 190.9 against 189.5).
   const uint32_t tiles = u.n_tiles * u.m_tiles, KS = p.K / 64u, units = u.T0 + (tiles - u.T0) * u.S;
   constexpr bool swiglu = EPI == P0P_EPI_SWIGLU;
 
@@ -220,6 +219,8 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     if (lane == 0) {
       Ring r(NS);
       bool ok = true;
+      grid_dependency_wait();
+      grid_launch_dependents();
       auto load2 = [&](uint32_t dst, const CUtensorMap* m, int x, int y, uint32_t bar) { if (PAIR) tma_load_2d_pair(dst, m, x, y, bar); else tma_load_2d(dst, m, x, y, bar); };
       auto load4 = [&](uint32_t dst, int c0, int c1, int c2, int c3, uint32_t bar) { if (PAIR) tma_load_4d_pair(dst, &mapX, c0, c1, c2, c3, bar); else tma_load_4d(dst, &mapX, c0, c1, c2, c3, bar); };
       const uint32_t nap = BT <= 64u ? 32u : 200u;                     // narrow tiles turn over quickly: poll their stages often
@@ -267,6 +268,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     if (ENC != P0P_ENC_F16 && lane == 0) {
       Ring q(NQ);
       bool ok = true;
+      grid_dependency_wait();
       const uint32_t last = (p.Nw >> 6) - 1u;                  // record tiles past the weight's end do not exist: their columns are never stored
       for (uint32_t unit = bid; unit < units && ok; unit += nblk) {
         const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t tile = un.tile, kb = un.kb, ke = un.ke;
@@ -296,6 +298,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     Ring r(NS), ar(NA);
     uint32_t tl = 0;
     bool ok = true;
+    grid_dependency_wait();
     for (uint32_t unit = bid; unit < units && ok; unit += nblk, tl++) {
       const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t kb = un.kb, ke = un.ke;
       const uint32_t buf = two_acc ? tl & 1u : 0u, par = two_acc ? (tl >> 1) & 1u : tl & 1u;
@@ -349,6 +352,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
     uint32_t tl = 0, pass = 0;
     bool ok = true;
     const bool vec = epilogue_vec_ok(p);
+    grid_dependency_wait();
     auto acc_free = [&](uint32_t b) { if (PAIR) mbar_arrive_cluster(cluster_addr(acc_empty + 8u * b, 0u)); else mbar_arrive(acc_empty + 8u * b); };
     for (uint32_t unit = bid; unit < units; unit += nblk, tl++) {
       const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t tile = un.tile, sp = un.sp;
@@ -431,6 +435,7 @@ __global__ void __launch_bounds__(U_THREADS, 1) k_gemm_umma(const UmmaP u, const
         }
       }
     };
+    grid_dependency_wait();
     for (uint32_t unit = bid; unit < units && ok; unit += nblk) {
       const UnitOf un = unit_of(u, unit, tiles, KS); const uint32_t n = un.ke - un.kb;
       for (uint32_t j0 = 0; j0 < n && ok; j0 += Q::KSUP, qr.next()) {
