@@ -119,6 +119,38 @@ def test_attention_split_keys(gpu, oracle, Hq, Hkv, Lq, Lk, mode, nvalid):
         for b in (qb, kb, vb, ob): gpu.free(b)
 
 
+@pytest.mark.parametrize("Lk,splits", [(60, False), (4096, True)])
+def test_attention_split_keys_special_values(gpu, Lk, splits):
+    """keys of score minus infinity weigh nothing (two whole key tiles of them: a share, or a split, that saw no other), a NaN among the valid keys
+    reaches every row that sees it and no other, an infinite value its own column"""
+    import p0pc0rn_kernels_b200 as P
+    rng = np.random.default_rng(5)
+    Hq, Hkv, nv = 12, 3, Lk - 3
+    q = rng.normal(0, 0.5, (Hq, 1, 128)); k = rng.normal(0, 0.5, (Hkv, Lk, 128)); v = rng.normal(0, 1, (Hkv, Lk, 128))
+    q[:, :, 0] = 0.5
+    gone = slice(128, 256) if splits else slice(16, 48)
+    k[0, gone, 0] = -np.inf
+    k[1, nv - 2, 3] = np.nan
+    v[2, 7, 5] = np.inf
+    q, k, v = (t.astype(np.float16) for t in (q, k, v))
+    k[:, nv:] = np.nan; v[:, nv:] = np.nan                                                    # past the valid length: never read
+    with np.errstate(invalid="ignore"):
+        s = np.einsum("hqd,hkd->hqk", q.astype(np.float64), np.repeat(k, Hq // Hkv, 0).astype(np.float64)[:, :nv]) / 128 ** 0.5
+        p = np.exp(s - s.max(2, keepdims=True)); p /= p.sum(2, keepdims=True)
+        want = np.einsum("hqk,hkd->qhd", p, np.repeat(v, Hq // Hkv, 0).astype(np.float64)[:, :nv])[0]
+    qb, kb, vb, ob = gpu.upload(q), gpu.upload(k), gpu.upload(v), gpu.buffer(Hq * 256)
+    try:
+        P.attention(gpu, {"q": {"buf": qb}, "k": {"buf": kb}, "v": {"buf": vb}, "o": {"buf": ob}, "Lq": 1, "Lk": Lk, "Hq": Hq, "Hkv": Hkv, "mode": 2, "nvalid": nv})
+        assert gpu.lastKernel == 16 and (gpu.lastPlan["S"] > 1) == splits
+        got = P.fromF16(gpu.read(ob).view(np.uint16)).reshape(Hq, 128)
+        assert np.isnan(got[4:8]).all() and np.isfinite(got[:4]).all()
+        assert np.array_equal(np.isposinf(got[8:]), np.isposinf(want[8:])) and np.isposinf(got[8:, 5]).all() and not np.isnan(got[8:]).any()
+        f = np.isfinite(want) & np.isfinite(got)
+        assert np.abs(got[f] - want[f]).max() <= 2e-2 * np.abs(want[f]).max()
+    finally:
+        for b in (qb, kb, vb, ob): gpu.free(b)
+
+
 def test_attention_split_keys_many_row_blocks(gpu):
     """more blocks of 64 query rows than a grid has in y or z (forced: the library's own choice for so many queries is the other kernel)"""
     import torch

@@ -565,6 +565,37 @@ def test_decode_few_tokens_share_the_columns(gpu, oracle, M, K):
         for b in (wb, xb, yb): gpu.free(b)
 
 
+@pytest.mark.parametrize("enc,M,N,K,KC", [("q4", 1, 64 * 420, 4096 + 256, 4096), ("q4", 1, 64 * 230, 8192 + 512, 4096), ("q8", 1, 64 * 420, 4096 + 768, 4096), ("q4", 2, 64 * 400, 2048 + 256, 2048)])
+def test_decode_long_blocks(gpu, oracle, enc, M, N, K, KC):
+    """the longest k-blocks, with a shorter last one.  Weights of this size are drawn as codes and scales; row tiles at the ends and spread
+    over the middle are compared, each with the decoded weights in 64 bits"""
+    O = oracle
+    rng = np.random.default_rng(7)
+    if enc == "q4":
+        q = rng.integers(0, 256, (N // 64, K // 32, 1024), dtype=np.uint8)
+        sm = np.stack([rng.uniform(0.002, 0.02, q.shape[:2] + (64,)), -rng.uniform(0.02, 0.1, q.shape[:2] + (64,))], -1).astype(np.float16).view(np.uint8).reshape(*q.shape[:2], 256)
+    else:
+        q = rng.integers(0, 256, (N // 64, K // 64, 4096), dtype=np.uint8)
+        sm = rng.uniform(0.0005, 0.002, q.shape[:2] + (64,)).astype(np.float16).view(np.uint8).reshape(*q.shape[:2], 128)
+    Wb = np.concatenate([q, sm], 2).ravel()
+    X = O.randn(M * K, 6); x = P().fromF16(P().toF16(X)).reshape(M, K).astype(np.float64)
+    wb, xb, yb = gpu.upload(Wb), gpu.upload(P().toF16(X)), gpu.buffer(M * N * 4)
+    try:
+        P().gemm(gpu, {"w": {"enc": CS.ENC_NAMES[enc], "buf": wb, "off": 0, "bytes": Wb.size, "rows": N, "cols": K}, "x": {"buf": xb}, "y": {"buf": yb}, "M": M, "N": N, "K": K, "epi": "f32", "kernel": "decode"})
+        plan = gpu.lastPlan
+        assert plan["KC"] == KC and K % KC and not plan["whole"], plan
+        got = gpu.read(yb, 0, M * N * 4).view(np.float32).reshape(M, N)
+        tiles = sorted({0, 1, N // 64 - 1, N // 64 - 2, *rng.integers(0, N // 64, 40)})
+        for t in tiles:
+            w = O.from_f16(O.dequant(CS.ENC_NAMES[enc], Wb, 64 * t, 64, K)[0]).reshape(64, K).astype(np.float64)
+            want = x @ w.T
+            # (the oracle's weights are rounded to fp16: 2^-11 relative per weight, uncorrelated)
+            assert np.linalg.norm(got[:, 64 * t:64 * t + 64] - want) <= 1e-3 * np.linalg.norm(want), t
+        assert np.isfinite(got).all()
+    finally:
+        for b in (wb, xb, yb): gpu.free(b)
+
+
 @pytest.mark.parametrize("case", DECODE, ids=lambda c: c["name"])
 def test_decode_kernel(gpu, oracle, case):
     """the decode-sized kernel (M <= 16: bulk-copy weight stream, raw codes on the tensor cores, split-K) against the oracle"""
@@ -744,6 +775,32 @@ def test_rowstats(gpu, oracle):
             got = gpu.read(sb, 16, rows * 8).view(np.float32)
             want = O.rowstats(X, rows, cols, rms=(mode == "rms"))
             assert np.allclose(got, want, rtol=2e-5, atol=1e-6)
+    finally:
+        gpu.free(xb); gpu.free(sb)
+
+
+@pytest.mark.parametrize("rows,cols,ld,c0,off", [
+    (5, 1001, 1001, 0, 0),          # columns not a multiple of four
+    (3, 8196, 8196, 0, 0),          # a row longer than the block's registers hold
+    (4, 8192, 8196, 4, 0),          # the longest row that they do hold, with a column offset
+    (7, 1000, 1003, 0, 0),          # rows not 16-byte aligned
+    (6, 512, 520, 2, 0),            # first column not 16-byte aligned
+    (2, 256, 256, 0, 4),            # the matrix itself not 16-byte aligned
+    (1, 64, 67, 0, 0),              # one row: its stride does not matter
+])
+def test_rowstats_forms(gpu, oracle, rows, cols, ld, c0, off):
+    """rows read as vectors held in registers, and rows read column by column (what the first form does not take)"""
+    O = oracle
+    X = (O.randn(rows * ld, 5) + 0.3).astype(np.float32)
+    xb, sb = gpu.upload(np.concatenate([np.full(off, 0x7F, np.uint8), X.view(np.uint8)])), gpu.buffer(rows * 8)
+    sub = X.reshape(rows, ld)[:, c0:c0 + cols].astype(np.float64)
+    try:
+        for mode in ("ln", "rms"):
+            P().rowstats(gpu, {"x": {"buf": xb, "off": off, "ld": ld, "c0": c0}, "rows": rows, "cols": cols, "mode": mode, "eps": 1e-6, "st": {"buf": sb}})
+            got = gpu.read(sb, 0, rows * 8).view(np.float32).reshape(rows, 2)
+            mean = sub.mean(1) if mode == "ln" else np.zeros(rows)
+            assert np.allclose(got[:, 0], mean, rtol=2e-5, atol=1e-6)
+            assert np.allclose(got[:, 1], 1.0 / np.sqrt(((sub - mean[:, None]) ** 2).mean(1) + 1e-6), rtol=2e-5)
     finally:
         gpu.free(xb); gpu.free(sb)
 

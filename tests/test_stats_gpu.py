@@ -29,7 +29,7 @@ def test_pixstats(gpu, oracle, V, C):
         for b in (xb, rb): gpu.free(b)
 
 
-@pytest.mark.parametrize("pix,C", [(64, 32), (100, 64), (1000, 128), (14720, 128), (200, 512), (129, 256)])
+@pytest.mark.parametrize("pix,C", [(64, 32), (100, 64), (1000, 128), (14720, 128), (200, 512), (129, 256), (64 * 257 + 9, 32), (64 * 600, 64)])
 def test_groupnorm_stats(gpu, oracle, pix, C):
     O = oracle
     X = O.to_f16(O.randn(pix * C, 5) * 2.0 + np.tile(np.linspace(-1, 1, C, dtype=np.float32), pix))
