@@ -164,8 +164,12 @@ extern "C" int p0p_gemm(p0p_ctx* c, const p0p_gemm_args* a_in, double* flops) {
   int rc = 0;
   // The streaming kernel wins up to 8 tokens (it never dequantises); from 9 on its second token group doubles its work and
   // the tensor-core kernel (narrow tiles, split-K) is faster on every shape measured.
-  // (5 to 8 tokens over a weight of up to 40 MB: the stream is too short to pay for the split-K reduction.  Measured at 5 and 8
-  // tokens, decode / tensor cores: 4096 x 4096 13.0, 15.2 / 11.5 us; 4096 x 14336 19.4, 22.6 / 18.8; 28672 x 4096 23.6, 26.7 / 31.1.)
+  // (5 to 8 tokens over up to 40 MB of codes: the stream is too short to pay for the split-K reduction.  Measured at 5 and 8 tokens,
+  // decode / tensor cores, us.  4-bit: 4096 x 4096 (10 MB) 11.2, 14.0 / 11.7; 8192 x 4096 (20 MB) 13.7, 16.4 / 15.5; 4096 x 14336 (35 MB)
+  // 19.9, 23.4 / 21.4; 16384 x 4096 (40 MB) 18.0, 20.8 / 17.2; 28672 x 4096 (70 MB) 25.2, 28.0 / 31.7.  8-bit: 4096 x 4096 (16 MB) 11.6, 13.7 / 11.8;
+  // 8192 x 4096 (32 MB) 14.5, 17.4 / 14.9; 4096 x 14336 (56 MB) 21.7, 25.5 / 20.9; 16384 x 4096 (64 MB) 20.2, 23.3 / 17.2; 28672 x 4096 (112 MB)
+  // 29.5, 33.5 / 30.1.  So the line is right at 8 tokens of 4-bit weights; at 5 the stream is 4 to 11 % ahead below 40 MB, and 8-bit weights
+  // would have it higher.)
   const bool dec_ok = decode_supported(p), um_ok = umma_supported(c, p);
   const uint64_t stream_bytes = (uint64_t)N * K * (a->enc == P0P_ENC_Q4 ? 5u : 8u) / 8u;
   const bool small_weight = p.M >= 5u && stream_bytes <= (40ull << 20);

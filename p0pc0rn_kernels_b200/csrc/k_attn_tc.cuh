@@ -3,15 +3,15 @@
 //   S = Q K^T   A = Q tile [128 q][128 d] (shared memory),  B = K tile [128 keys][128 d] (shared memory, K-major: d contiguous)
 //   O += P V    A = P tile [128 q][128 keys] (tensor memory), B = V tile [128 keys][128 d] (shared memory, MN-major: d, the N of
 //               this product, is contiguous).  V is read as it lies; a transposed copy (so that B would be K-major) was a pass of
-//               its own over V (32:8 heads, 1000 causal tokens: 26.7 -> 24.6 us a call without it)
+//               its own over V (32:8 heads, 1000 causal tokens: 26.7 -> 24.6 us a call, this and two softmax threads per row together)
 // One block = two tiles of 128 queries of one head that share every K / V tile (or one tile: see attn_plan).  Tensor memory (512 columns x 128 lanes):
 // S of tile A | S of tile B | O of tile A | O of tile B, 128 fp32 columns each; lane = query row.  P (fp16, two keys per
 // column) is written over the first 64 columns of its S, which is free once the softmax threads hold the row.
-// P is handed over in two halves of 64 keys, so the first half of PV runs under the second half's exponentials.
 // Roles: warp 0 loads tiles by tensor-map copies into a ring of 32-KB slots (K0 V0 K1 V1 ...); warp 1 issues the
 // multiplies in the order  PV_A(j) QK_A(j+1) PV_B(j) QK_B(j+1), so that while the softmax of one tile runs the tensor
-// cores work on the other; warps 2-5 are the softmax of tile A, warps 6-9 of tile B: one thread per query row, the whole
-// row of 128 scores in registers (no shuffles).  The running maximum is only raised when it grew by more than 2^8: until
+// cores work on the other; warps 2-9 are the softmax of tile A, warps 10-17 of tile B: two threads per query row, 64 scores each
+// in registers; the two tell each other their row maximum (and at the end their sum) through shared memory, and P is handed to
+// the multiplies once both have stored their half.  The running maximum is only raised when it grew by more than 2^8: until
 // then P is at most 256 (fine in fp16) and O needs no rescaling, which is a pass over tensor memory.  "S(j+1) ready"
 // implies "PV(j) done" (a commit covers every earlier multiply), so the softmax threads may rescale O when they hold S.
 #pragma once
@@ -59,7 +59,9 @@ constexpr uint32_t ATC_SMEM = 1024u + (2u + ATC_SLOTS) * ATC_TILE + 256u + 4096u
 
 #ifndef ATC_EMU
 #define ATC_EMU 6          // of every 16 pairs of scores, how many take their exponential on the FMA pipe instead of the MUFU
-                           // (24 heads x 3600 x 3600: 0 -> 193 us, 4 -> 186, 6 -> 183, 8 -> 207)
+                           // (with two threads per query row, in long runs; 24 heads x 3600 x 3600 and 32:8 heads x 1000
+                           // causal: 0 185.1, 20.95 us; 4 188.2, 20.50; 5 187.6, 20.41; 6 191.1, 20.71; 7 190.8, 20.75; 8 205.5, 22.72.
+                           // 6 was the best with one thread per row: 0 193, 4 186, 6 183, 8 207)
 #endif
 
 __device__ __forceinline__ float atc_ex2(float x) { float y; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x)); return y; }
@@ -301,8 +303,9 @@ __global__ void __launch_bounds__(ATC_THREADS, 1) k_attn_tc(const AttnTcP p, con
 // How a head's T tiles of 128 queries are cut into blocks.  Two-tile blocks are the efficient ones (K / V tiles shared, the
 // softmax of one tile hidden behind the multiplies of the other), but blocks are handed to SMs whole: 15 two-tile blocks
 // per head x 24 heads on 148 SMs is 2.4 rounds, of which the third is mostly idle.  One-tile blocks cost ATC_SINGLE_COST of a
-// two-tile block (measured: with nothing to overlap its softmax with, one tile takes 0.85 of the time of two) and fill that
-// last round.  The plan simulates the hardware's in-order hand-out for every split and keeps
+// two-tile block (nothing overlaps their softmax: 28 key tiles, 148 heads, 54.6 us against 64.3 in a short run; 50.8 against 72.6, 0.70, in a
+// long one, where the power limit slows the denser blocks) and fill that last round.  (24 heads x 3600: 1 to 7 one-tile blocks per
+// head within 0.5 % of one another in long runs, 9 are 14 % slower.)  The plan simulates the hardware's in-order hand-out for every split and keeps
 // the shortest; cost of a block = its key tiles (they differ under the causal mask).
 constexpr double ATC_SINGLE_COST = 0.85;
 inline void attn_plan(uint32_t Lq, uint32_t Lk, uint32_t Hq, uint32_t mode, uint32_t nvalid, uint32_t sms, uint32_t& np, uint32_t& ns) {

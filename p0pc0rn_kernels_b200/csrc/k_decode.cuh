@@ -186,13 +186,6 @@ template <uint32_t O> __device__ __forceinline__ uint4 lds128_if(uint32_t a, uin
   return v;
 }
 
-// (a & mask) | magic in ONE instruction (left to the compiler this becomes two)
-__device__ __forceinline__ uint32_t and_or(uint32_t a, uint32_t mask, uint32_t magic) {
-  uint32_t d;
-  asm("lop3.b32 %0, %1, %2, %3, 0xEA;" : "=r"(d) : "r"(a), "r"(mask), "r"(magic));
-  return d;
-}
-
 // D = A * B + C with C given separately (the correction terms ride in on C)
 __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1, const float (&c)[4]) {
   asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
@@ -201,7 +194,7 @@ __device__ __forceinline__ void mma_16816(float (&d)[4], uint32_t a0, uint32_t a
 }
 
 // per-lane constants of the consumer loop
-struct DLane { uint32_t MLO, MHI, MAGIC; uint32_t on0, on1; bool one; };
+struct DLane { uint32_t MLO, MHI; uint32_t on0, on1; bool one; };
 
 // one q4 record (64 rows x 32 k) of this warp's share of a stage: R is its index in the share.  ta: sums of s * acc (to be
 // scaled by 2^24), tb: sums of mn * Sx.
@@ -376,7 +369,7 @@ __global__ void __launch_bounds__(D_THREADS, D_PER_SM) k_decode_stream(const Dec
   const uint32_t cts_l = smem_u32(cts) + (from * (MP / 2) + tp) * 8u;
   float* comb_l = comb + (rg * 32u + lane) * (4 * NF);
   DLane L;
-  L.MLO = 0x000f000fu; L.MHI = 0x00f000f0u; L.MAGIC = 0x64006400u;      // (masks live in registers: as immediates each AND would cost a constant load)
+  L.MLO = 0x000f000fu; L.MHI = 0x00f000f0u;      // (masks live in registers: as immediates each AND would cost a constant load)
   L.on0 = g < p.M ? 1u : 0u; L.on1 = g + 8u < p.M ? 1u : 0u;            // does this lane's token column exist?
   L.one = p.M == 1u;                                                     // a single token: only the accumulators of token 0 are kept up
   uint32_t s = 0, ph = 0, cur_kb = 0xffffffffu;

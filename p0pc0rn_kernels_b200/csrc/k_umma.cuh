@@ -133,7 +133,7 @@ constexpr uint32_t U_NX_MAX = 8;         // most stages of the token ring
 // Three producers feed the multiply, each through a ring of stages with a "ready" and a "free" mbarrier per stage:
 //   X  token tiles (and fp16 weight tiles), NS stages of shared memory of KW sub-tiles each, filled by TMA;
 //   Q  quantised records, NQ stages of shared memory, filled by bulk copies (KSUP k-steps each, a multiple of KW);
-//   A  dequantised weight operand: NA stages of KW 32-column sub-stages of tensor memory (NA * KW <= 4), filled by the
+//   A  dequantised weight operand: NA stages of KW 32-column sub-stages of tensor memory (all the columns behind the accumulators, 8 stages at most), filled by the
 //      dequantisation warps.
 // Wide tiles are bound by the multiplies, and there every instruction the issuing warp runs between two multiplies shows in the
 // total: X and A then advance in lock step (NA = NS) and SHARE their barriers - one wait and one commit per step.  Narrow tiles
@@ -144,8 +144,8 @@ constexpr uint32_t U_NX_MAX = 8;         // most stages of the token ring
 // in turn (each step's one or two k-steps by one group), except in the lock-step 128-k variant, whose two operand stages
 // leave no room for that: there group g converts sub-step g of every step, both side by side.  The warps that wait are
 // parked by the hardware (mbar_try), not spinning beside the ones that work.
-// KW and LOCK are compile-time (four variants exist: (1, lock), (2, lock), (2, separate), (4, separate; 4-bit weights)): the issuing warp's loop is the
-// critical path of wide tiles and must not carry run-time choices.
+// KW, LOCK and PAIR are compile-time (quantised weights: (1, lock), (2, lock), (2, separate), (4, separate) and (1, lock, pair); fp16
+// weights: (1, lock), alone and as a pair): the issuing warp's loop is the critical path of wide tiles and must not carry run-time choices.
 //
 // PAIR: two blocks of a cluster (the two SMs of a TPC) compute one tile of 256 columns x BT tokens with tcgen05's cta_group::2.
 // Each block holds 128 weight rows - its own operand ring and accumulator, as without PAIR - but only HALF of the token tile: a
