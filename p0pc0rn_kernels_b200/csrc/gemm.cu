@@ -164,15 +164,18 @@ extern "C" int p0p_gemm(p0p_ctx* c, const p0p_gemm_args* a_in, double* flops) {
   int rc = 0;
   // The streaming kernel wins up to 8 tokens (it never dequantises); from 9 on its second token group doubles its work and
   // the tensor-core kernel (narrow tiles, split-K) is faster on every shape measured.
-  // (5 to 8 tokens over up to 40 MB of codes: the stream is too short to pay for the split-K reduction.  Measured at 5 and 8 tokens,
-  // decode / tensor cores, us.  4-bit: 4096 x 4096 (10 MB) 11.2, 14.0 / 11.7; 8192 x 4096 (20 MB) 13.7, 16.4 / 15.5; 4096 x 14336 (35 MB)
-  // 19.9, 23.4 / 21.4; 16384 x 4096 (40 MB) 18.0, 20.8 / 17.2; 28672 x 4096 (70 MB) 25.2, 28.0 / 31.7.  8-bit: 4096 x 4096 (16 MB) 11.6, 13.7 / 11.8;
-  // 8192 x 4096 (32 MB) 14.5, 17.4 / 14.9; 4096 x 14336 (56 MB) 21.7, 25.5 / 20.9; 16384 x 4096 (64 MB) 20.2, 23.3 / 17.2; 28672 x 4096 (112 MB)
-  // 29.5, 33.5 / 30.1.  So the line is right at 8 tokens of 4-bit weights; at 5 the stream is 4 to 11 % ahead below 40 MB, and 8-bit weights
-  // would have it higher.)
+  // 5 to 8 tokens over a short stream: it does not pay for the split-K reduction.  The line lies at 40 MB of codes for 7 and 8 tokens; for 5
+  // and 6 at 16 MB, and at 40 only where the column tiles fill one round of the SMs, so that the tensor-core kernel need not split k
+  // either.  Measured at 5, 6, 7, 8 tokens, decode / tensor cores, us.  4-bit: 4096 x 4096 (10 MB) 11.2, -, -, 14.0 / 11.7; 8192 x 4096 (20 MB) 13.7,
+  // 14.3, 15.4, 16.4 / 15.4; 4096 x 14336 (35 MB) 19.9, 21.5, 22.5, 23.4 / 21.4; 16384 x 4096 (40 MB, 128 tiles) 18.0, 19.2, 20.2, 20.8 / 17.2;
+  // 28672 x 4096 (70 MB) 25.2, 26.3, 27.4, 28.0 / 31.7.  8-bit: 4096 x 4096 (16 MB) 11.6, -, -, 13.7 / 11.8; 6144 x 4096 (24 MB) 13.7, 14.6, 15.4,
+  // 16.1 / 14.7; 8192 x 4096 (32 MB) 14.5, 15.3, 16.1, 17.4 / 15.0; 4096 x 14336 (56 MB) 21.7, 22.9, 24.2, 25.5 / 20.9; 16384 x 4096 (64 MB) 20.2, 21.3,
+  // 22.4, 23.3 / 17.2; 28672 x 4096 (112 MB) 29.5, 31.4, 32.5, 33.5 / 30.1: for 8-bit weights the line could lie higher.
   const bool dec_ok = decode_supported(p), um_ok = umma_supported(c, p);
   const uint64_t stream_bytes = (uint64_t)N * K * (a->enc == P0P_ENC_Q4 ? 5u : 8u) / 8u;
-  const bool small_weight = p.M >= 5u && stream_bytes <= (40ull << 20);
+  const uint32_t col_tiles = (N + 127u) / 128u, sms = (uint32_t)c->prop.multiProcessorCount;
+  const bool one_round = col_tiles <= sms && col_tiles * 4u > sms * 3u;
+  const bool small_weight = p.M >= 5u && stream_bytes <= ((p.M >= 7u || one_round ? 40ull : 16ull) << 20);
   if (want == P0P_K_DECODE || (want == P0P_K_AUTO && dec_ok && ((p.M <= 8u && !small_weight) || !um_ok))) {
     if (!dec_ok) return fail(c, -9, "gemm: the decode kernel does not take this configuration");
     rc = launch_decode(c, p); used = P0P_K_DECODE;

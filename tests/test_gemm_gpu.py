@@ -596,6 +596,26 @@ def test_decode_long_blocks(gpu, oracle, enc, M, N, K, KC):
         for b in (wb, xb, yb): gpu.free(b)
 
 
+@pytest.mark.parametrize("enc,N,K,M,family", [
+    ("q4", 4096, 4096, 4, "decode"), ("q4", 4096, 4096, 5, "umma"),                                              # 10 MB of codes
+    ("q4", 8192, 4096, 5, "decode"), ("q4", 8192, 4096, 6, "decode"), ("q4", 8192, 4096, 7, "umma"),              # 20 MB, 64 column tiles
+    ("q8", 6144, 4096, 6, "decode"), ("q8", 6144, 4096, 8, "umma"),                                              # 24 MB
+    ("q4", 16384, 4096, 5, "umma"),                                                                              # 40 MB, 128 column tiles: one round
+    ("q4", 17408, 4096, 8, "decode"),                                                                            # above 40 MB
+])
+def test_kernel_choice_of_few_tokens(gpu, enc, N, K, M, family):
+    """which kernel serves 4 to 8 tokens, on both sides of each line"""
+    nb = N * K * 5 // 8 if enc == "q4" else N * K * 33 // 32
+    w, x, y = gpu.buffer(nb), gpu.buffer(M * K * 2), gpu.buffer(M * N * 2)
+    try:
+        P().gemm(gpu, {"w": {"enc": CS.ENC_NAMES[enc], "buf": w, "off": 0, "bytes": nb, "rows": N, "cols": K}, "x": {"buf": x}, "y": {"buf": y}, "M": M, "N": N, "K": K})
+        assert P()._lib.KERNEL_NAMES[gpu.lastKernel] == family
+        assert not gpu.read(y).any()
+    finally:
+        for b in (w, x, y): gpu.free(b)
+        gpu.drainPool()
+
+
 @pytest.mark.parametrize("case", DECODE, ids=lambda c: c["name"])
 def test_decode_kernel(gpu, oracle, case):
     """the decode-sized kernel (M <= 16: bulk-copy weight stream, raw codes on the tensor cores, split-K) against the oracle"""
