@@ -278,7 +278,7 @@ def run_configs(args, P, torch, gpu, stream, dev, pk, rank, world):
             def call(): P.attention(gpu, {"q": {"buf": q}, "k": {"buf": k}, "v": {"buf": v}, "o": {"buf": o}, "Lq": L, "Lk": L, "Hq": H, "Hkv": H, "mode": 0})
             ms = graph_time(call, max(3, min(args.steps, 20)))
             fl = 4.0 * L * L * 128 * H
-            print(json.dumps({"config": "attention after dit_qkv (24 heads x 3600 tokens x 128, no mask)", "family": {16: "split-key mma.sync attention", 17: "tcgen05 flash attention (V transposed by a pre-pass, inside the timed call)"}.get(gpu.lastKernel), "ms": ms,
+            print(json.dumps({"config": "attention after dit_qkv (24 heads x 3600 tokens x 128, no mask)", "family": {16: "split-key mma.sync attention", 17: "tcgen05 flash attention"}.get(gpu.lastKernel), "ms": ms,
                               "TFLOP/s": fl / (ms * 1e-3) / 1e12, "frac_tensor": fl / (ms * 1e-3) / 1e12 / pk["tensor"]}), flush=True)
             for b in (q, k, v, o): gpu.free(b)
         elif name == "conv3":
@@ -343,11 +343,12 @@ def run_configs(args, P, torch, gpu, stream, dev, pk, rank, world):
 
 
 # DRAM bytes per launch of the dominant kernel (dram__bytes_read.sum + dram__bytes_write.sum of one ncu capture of this
-# command, see profiles/), keyed by (call, tokens, kernel family, ranks, kernel plan).  A launch whose plan differs from the
+# command, see profiles/), keyed by (call, tokens, kernel family, ranks), with the plan it was taken at.  A launch whose plan differs from the
 # captured one reports null rather than a stale figure.
 TRAFFIC = {
     # dram__bytes_read.sum + dram__bytes_write.sum of the k_gemm_umma launch of the gate/up call (the norm pre-pass adds 12.6 MB)
-    ("gate_up", 512, "umma", 1): {"bytes": 81271296.0, "plan": "448 tiles of 128 x 256, last round split along K", "captured_at": "71786ec"},
+    ("gate_up", 512, "umma", 1): {"bytes": 81580288.0, "plan": "224 pair tiles of 256 columns x 256 tokens, last round split along K",
+                                  "cut": {"PAIR": 1, "BT": 256, "S": 4, "T0": 222}, "captured_at": "db7b18b"},
 }
 
 
@@ -557,6 +558,7 @@ def run_block(args, P, torch, dist, gpu, stream, dev, pk, rank, world, local):
     ms, per_round, gs_head = timed(M, args.steps, max(3, args.warmup), max(1, args.rounds))
     n_launch = launches["n"]
     gu_ms, gu_kernel = kernel_ms(M, "gate_up", max(20, min(100, args.steps)))
+    gu_plan = gpu.lastPlan
     # keep the GPU under the same load until the sampler (200 ms period) has a few readings of the clocks.  The replay count
     # comes from `ms`, which was all-reduced above: the same on every rank (each replay holds cross-rank barriers).
     n_load = int(min(20000, max(50, 1.2 / (ms * 1e-3))))
@@ -730,6 +732,7 @@ def run_block(args, P, torch, dist, gpu, stream, dev, pk, rank, world, local):
     gu_flops = 2.0 * M * (2 * ffl) * HID
     fam_name = P._lib.KERNEL_NAMES.get(gu_kernel)
     tr = TRAFFIC.get(("gate_up", M, fam_name, world))
+    if tr and any(gu_plan.get(k) != v for k, v in tr["cut"].items()): tr = None
     roof = {"bound": "tensor", "achieved": gu_flops / (gu_ms * 1e-3) / 1e12, "peak": pk["tensor"], "unit": "TFLOP/s", "traffic": tr["bytes"] if tr else None,
             "traffic_source": f"ncu capture at {tr['captured_at']} ({tr['plan']})" if tr else None,
             "kernel": f"gate/up GEMM call ({fam_name} family: norm pre-pass + tensor-core kernel), M={M}", "ms_per_launch": gu_ms, "peak_source": pk["src"] + " (burst cuBLAS bf16)"}

@@ -43,7 +43,7 @@ constexpr int D_PER_SM = 3;                 // blocks an SM's registers hold (28
 // How the two warps of a row group divide the stages: in turn, so that what a warp pays per stage beside its records (the barrier,
 // addresses, scales) is paid half as often; or a half of each, which is the faster form where the records outweigh that (4-bit
 // weights, 5 tokens and more: 8 x 28672 x 4096 26.7 us against 28.7 in turn).  In turn, with k-blocks of 4096 for one token:
-// 1 x 16384 x 16384 38.2 -> 33.6 us, 1 x 28672 x 4096 20.4 -> 17.2.
+// 1 x 16384 x 16384 38.2 -> 35.8 us, 1 x 28672 x 4096 20.4 -> 17.6.
 template <int ENC, int MP> constexpr bool D_TURNS = ENC == P0P_ENC_Q8 || MP < 8;
 // Stages of the ring: in turn an EVEN number, so that a slot always belongs to the same one of the two warps.  (With an odd number a
 // warp meets a slot in every second of its phases only, and a wait by parity cannot tell a phase from the one two before it.)
